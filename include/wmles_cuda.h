@@ -136,8 +136,8 @@ typedef struct {
     const wm_inflow* inflow;      /* NULL if no synthetic-turbulence inflow */
     wm_sponge sponge;
     int tile;                 /* stage-kernel tile shape id (0 = 8x32, 1 = 16x16, 2 = 4x32,
-                                 3 = 16x32, mixed form only); -1 = automatic: 0 for FP64,
-                                 3 for the mixed form */
+                                 3 = 16x32, mixed form only); -1 = automatic: a shape per
+                                 block from its extents */
     int chunk;                /* planes per CTA along i, 0 = automatic */
 } wm_case_desc;
 

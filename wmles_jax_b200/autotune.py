@@ -1,7 +1,8 @@
 """Tile-shape autotuner for the fused stage kernel.
 
 The stage kernel marches a TJ x TK column of cells along i (tile ids: 0 = 8x32, 1 = 16x16,
-2 = 4x32, 3 = 16x32, the last built for the mixed form only).  Which shape is fastest depends
+2 = 4x32, 3 = 16x32, the last built for the mixed form only; -1 = a shape per block from its
+extents, the default).  Which shape is fastest depends
 on the grid extents (partial tiles at the j/k edges, waves of CTAs over the SMs), on the
 precision (registers and shared memory decide CTAs per SM) and on the scheme.  ``tune``
 measures it: for each candidate tile it builds the cases with that tile, advances them
@@ -21,8 +22,8 @@ import threading
 
 import numpy as np
 
-TILE_SHAPES = {0: (8, 32), 1: (16, 16), 2: (4, 32), 3: (16, 32)}
-CANDIDATES = {"fp64": (0, 1, 2), "mixed": (0, 1, 2, 3)}
+TILE_SHAPES = {-1: None, 0: (8, 32), 1: (16, 16), 2: (4, 32), 3: (16, 32)}
+CANDIDATES = {"fp64": (-1, 0, 1, 2), "mixed": (-1, 0, 1, 2, 3)}
 _LOCK = threading.Lock()
 
 
@@ -136,7 +137,7 @@ def tune(cases, precision="mixed", tiles=None, steps=20, warmup=3, use_cache=Tru
         del solvers, bufs, dts, qa, qb
     best = pick(timings)
     if use_cache:
-        store(key, {"tile": best, "tile_shape": list(TILE_SHAPES[best]),
+        store(key, {"tile": best, "tile_shape": TILE_SHAPES[best] and list(TILE_SHAPES[best]),
                     "ms_per_step": {str(k): v for k, v in timings.items()}, "steps": steps}, path)
     return best, timings
 

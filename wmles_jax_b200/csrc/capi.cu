@@ -178,10 +178,17 @@ struct View {
     std::vector<BlockDev> hb;
     std::vector<CaseDev> hc;
     std::vector<WallDev> hw;
-    std::vector<Tile> tiles;             // stage work list: (j,k) columns of every block, cut along i
-    std::vector<int> cta_first;          // balanced split: CTA c runs tiles [cta_first[c], cta_first[c+1])
+    // stage work lists, of the general blocks and of those extruded along k (each one launch): the
+    // blocks' (j,k) columns, cut along i
+    struct Work {
+        std::vector<int> blocks;         // view blocks
+        std::vector<Tile> tiles;
+        std::vector<int> cta_first;      // balanced split: CTA c runs tiles [cta_first[c], cta_first[c+1])
                                          // (empty: one tile per CTA)
-    int* d_cta_first = nullptr;
+        Tile* d_tiles = nullptr;
+        int* d_cta_first = nullptr;
+        int ctas() const { return cta_first.empty() ? (int)tiles.size() : (int)cta_first.size() - 1; }
+    } work[2];
     std::vector<int> case_block_start;
     std::vector<int> cmf_slot_start, case_slot_start;   // constant-mass-flux partial slots
     std::vector<GhostSeg> seg_rhs, seg_all;
@@ -189,7 +196,6 @@ struct View {
     BlockDev* d_blocks = nullptr;
     CaseDev* d_cases = nullptr;
     WallDev* d_walls = nullptr;
-    Tile* d_tiles = nullptr;
     int* d_case_slot_start = nullptr;
     GhostSeg *d_seg_rhs = nullptr, *d_seg_all = nullptr;
     double *cmf_part = nullptr, *cmf_delta = nullptr;
@@ -302,8 +308,20 @@ int validate(const wm_case_desc* d) {
     return WM_OK;
 }
 
+// (j,k) tile columns of a block
+long long columns(const BlockDev& B) {
+    return (long long)((B.n[1] + B.tj - 1) / B.tj) * ((B.n[2] + B.tk - 1) / B.tk);
+}
+
+// the tile of a block's column at (j0, k0) over planes [i0, i1)
+Tile make_tile(const BlockDev& B, int b, int j0, int k0, int i0, int i1) {
+    const int colk = (B.n[2] + B.tk - 1) / B.tk;
+    return Tile{b, j0, k0, i0, i1, std::min(B.tj, B.ng + B.n[1] - j0), std::min(B.tk, B.ng + B.n[2] - k0),
+                ((j0 - B.ng) / B.tj) * colk + (k0 - B.ng) / B.tk};
+}
+
 // planes per stage-kernel CTA: wave quantisation against the chunk prologue cost
-int choose_chunk(const std::vector<BlockDev>& hb, const StageOpts& opts, int tj, int tk, int requested) {
+int choose_chunk(const std::vector<BlockDev>& hb, const std::vector<int>& blocks, const StageOpts& opts, int requested) {
     if (requested > 0) return requested;
     int sms = 148, dev = 0;
     cudaGetDevice(&dev);
@@ -312,17 +330,14 @@ int choose_chunk(const std::vector<BlockDev>& hb, const StageOpts& opts, int tj,
     if (occ < 1) occ = 1;
     const long long slots = (long long)sms * occ;
     int nimax = 0;
-    for (const BlockDev& B : hb) nimax = std::max(nimax, B.n[0]);
+    for (int b : blocks) nimax = std::max(nimax, hb[b].n[0]);
     double best = 1e300;
     int best_ic = nimax;
-    for (int ic = 4; ic <= std::max(4, nimax); ++ic) {
+    for (int ic = 1; ic <= nimax; ++ic) {
         long long ctas = 0;
-        for (const BlockDev& B : hb) {
-            const long long jk = (long long)((B.n[1] + tj - 1) / tj) * ((B.n[2] + tk - 1) / tk);
-            ctas += jk * ((B.n[0] + ic - 1) / ic);
-        }
+        for (int b : blocks) ctas += columns(hb[b]) * ((hb[b].n[0] + ic - 1) / ic);
         const long long waves = (ctas + slots - 1) / slots;
-        const double cost = double(waves) * (std::min(ic, nimax) + 3);
+        const double cost = double(waves) * (std::min(ic, nimax) + SEG_PLANES);
         if (cost < best - 1e-9) { best = cost; best_ic = ic; }
     }
     return best_ic;
@@ -337,86 +352,121 @@ int stage_slots(const StageOpts& opts) {
     return sms * (occ < 1 ? 1 : occ);
 }
 
-// wave split, for views with fewer (j,k) columns than resident CTAs and one plane count n0:
+// wave split, for work lists with fewer (j,k) columns than resident CTAs and one plane count n0:
 // every column is cut at the same planes into q = slots / C equal chunks over [0, n0 - x)
 // (q full waves, all columns in lockstep, so halo reads of neighbouring columns hit L2), and
 // the last x planes of every column go to the r = slots - q C CTAs left over, each taking
 // the tail of columns m, m + r, m + 2 r, ... in turn (again in lockstep).  x balances the
-// chunk length against the tail CTAs' segments; each segment costs `prologue` planes more.
-// Returns the slowest CTA's cost in planes (1e300 when the split does not apply).
-double build_waves(View* v, int tj, int tk, int slots, double prologue) {
+// chunk length against the tail CTAs' segments (split_planes); 0: no such split is the cheapest
+void build_waves(const std::vector<BlockDev>& hb, View::Work* v, int slots) {
     struct Col { int b, j0, k0; };
     std::vector<Col> cols;
-    const int n0 = v->hb[0].n[0];
-    for (int b = 0; b < v->nblocks; ++b) {
-        const BlockDev& B = v->hb[b];
-        if (B.n[0] != n0) return 1e300;
-        for (int j0 = B.ng; j0 < B.ng + B.n[1]; j0 += tj)
-            for (int k0 = B.ng; k0 < B.ng + B.n[2]; k0 += tk) cols.push_back(Col{b, j0, k0});
+    const int n0 = hb[v->blocks[0]].n[0];
+    for (int b : v->blocks) {
+        const BlockDev& B = hb[b];
+        if (B.n[0] != n0) return;
+        for (int j0 = B.ng; j0 < B.ng + B.n[1]; j0 += B.tj)
+            for (int k0 = B.ng; k0 < B.ng + B.n[2]; k0 += B.tk) cols.push_back(Col{b, j0, k0});
     }
     const int C = (int)cols.size();
-    const int q = slots / C, r = slots - q * C;
-    if (q < 1 || r < 1) return 1e300;
-    const int m = (C + r - 1) / r;                 // tail segments of the busiest tail CTA
-    double best = 1e300;
-    int bx = 0;
-    for (int x = 16; x < n0 / 2; ++x) {           // tail segments of at least 16 planes
-        const double main_cost = std::ceil(double(n0 - x) / q) + prologue;
-        const double tail_cost = m * (x + prologue);
-        const double cost = std::max(main_cost, tail_cost);
-        if (cost < best - 1e-9) { best = cost; bx = x; }
-    }
-    if (bx == 0) return 1e300;
-    const int L = (n0 - bx + q - 1) / q;
+    int x = 0;
+    split_planes(C, n0, slots, nullptr, &x);
+    if (x == 0) return;
+    const int q = slots / C, r = slots - q * C, L = (n0 - x + q - 1) / q;
     v->tiles.clear();
     v->cta_first.assign(1, 0);
     for (int w = 0; w < q; ++w)
         for (const Col& c : cols) {
-            const int ng = v->hb[c.b].ng;
-            const int lo = w * L, hi = std::min((w + 1) * L, n0 - bx);
-            if (hi > lo) v->tiles.push_back(Tile{c.b, c.j0, c.k0, ng + lo, ng + hi});
+            const int ng = hb[c.b].ng;
+            const int lo = w * L, hi = std::min((w + 1) * L, n0 - x);
+            if (hi > lo) v->tiles.push_back(make_tile(hb[c.b], c.b, c.j0, c.k0, ng + lo, ng + hi));
             v->cta_first.push_back((int)v->tiles.size());
         }
     for (int t = 0; t < r; ++t) {
         for (int c = t; c < C; c += r) {
-            const int ng = v->hb[cols[c].b].ng;
-            v->tiles.push_back(Tile{cols[c].b, cols[c].j0, cols[c].k0, ng + n0 - bx, ng + n0});
+            const int ng = hb[cols[c].b].ng;
+            v->tiles.push_back(make_tile(hb[cols[c].b], cols[c].b, cols[c].j0, cols[c].k0, ng + n0 - x, ng + n0));
         }
         v->cta_first.push_back((int)v->tiles.size());
     }
-    return best;
 }
 
 // constant-mass-flux partial slots of a view: one per (column, interior plane) of each block,
 // independent of how the columns are cut into CTAs
-void cmf_slots(View* v, int tj, int tk) {
+void cmf_slots(View* v) {
     v->cmf_slot_start.assign(1, 0);
     for (int b = 0; b < v->nblocks; ++b) {
         const BlockDev& B = v->hb[b];
-        const int cols = ((B.n[1] + tj - 1) / tj) * ((B.n[2] + tk - 1) / tk);
-        v->cmf_slot_start.push_back(v->cmf_slot_start.back() + cols * B.n[0]);
+        v->cmf_slot_start.push_back(v->cmf_slot_start.back() + (int)columns(B) * B.n[0]);
     }
     v->case_slot_start.clear();
     for (int c = 0; c <= v->ncases; ++c) v->case_slot_start.push_back(v->cmf_slot_start[v->case_block_start[c]]);
 }
 
 // chunked split: every column cut into chunks of ic planes, one chunk per CTA
-void build_tiles(View* v, int tj, int tk, int ic) {
+void build_tiles(const std::vector<BlockDev>& hb, View::Work* v, int ic) {
     v->tiles.clear();
     v->cta_first.clear();
-    for (int b = 0; b < v->nblocks; ++b) {
-        const BlockDev& B = v->hb[b];
+    for (int b : v->blocks) {
+        const BlockDev& B = hb[b];
         const int ng = B.ng;
         for (int i0 = ng; i0 < ng + B.n[0]; i0 += ic)
-            for (int j0 = ng; j0 < ng + B.n[1]; j0 += tj)
-                for (int k0 = ng; k0 < ng + B.n[2]; k0 += tk)
-                    v->tiles.push_back(Tile{b, j0, k0, i0, std::min(i0 + ic, ng + B.n[0])});
+            for (int j0 = ng; j0 < ng + B.n[1]; j0 += B.tj)
+                for (int k0 = ng; k0 < ng + B.n[2]; k0 += B.tk)
+                    v->tiles.push_back(make_tile(B, b, j0, k0, i0, std::min(i0 + ic, ng + B.n[0])));
     }
 }
 
 bool same_opts(const StageOpts& a, const StageOpts& b) {
     return a.precision == b.precision && a.scheme == b.scheme && a.kep_order == b.kep_order &&
            a.limiter == b.limiter && a.sgs == b.sgs && a.tile == b.tile;
+}
+
+// Row and k tables of a block extruded along k (left null otherwise): its stage kernel takes the
+// metrics of a row from shared memory instead of loading 21 per face and 20 per gradient
+// record, and leaves out the products with their zero components (stage.cu).  The factor per k of
+// the i- and j-face areas is taken from the first interior row's i face (their larger component).
+// The tables reproduce the metrics to a few units in the last place (tolerance 16).
+int extruded_tables(wm_case* c, BlockDev& B, int precision) {
+    B.rows = B.ktab = nullptr;
+    B.rows32 = B.ktab32 = nullptr;
+    const int Nk = B.N[2], k0 = B.ng;
+    const size_t n = (size_t)B.ncell, row = ((size_t)B.ng * B.N[1] + B.ng) * Nk;
+    std::vector<double> sx(Nk), sy(Nk), id(Nk), kt(2 * (size_t)Nk);
+    CK(cudaMemcpy(sx.data(), B.met + WM_MET_SIX * n + row, sizeof(double) * Nk, cudaMemcpyDeviceToHost));
+    CK(cudaMemcpy(sy.data(), B.met + WM_MET_SIY * n + row, sizeof(double) * Nk, cudaMemcpyDeviceToHost));
+    CK(cudaMemcpy(id.data(), B.met + WM_MET_IDK * n + row, sizeof(double) * Nk, cudaMemcpyDeviceToHost));
+    const std::vector<double>& s = std::fabs(sx[k0]) >= std::fabs(sy[k0]) ? sx : sy;
+    for (int k = 0; k < Nk; ++k) {
+        kt[2 * k] = s[k] / s[k0];
+        kt[2 * k + 1] = id[k];
+        if (!(kt[2 * k] > 0.0)) return WM_OK;
+    }
+    Owner tmp;
+    double* d_kt = nullptr;
+    int *flag = nullptr, ok = 1;
+    int r;
+    if ((r = tmp.upload(&flag, &ok, 1))) return r;
+    if ((r = c->mem.upload(&d_kt, kt.data(), kt.size()))) return r;
+    CK(launch_ext_check(B.met, B.N, B.ng, k0, d_kt, 16 * 2.220446049250313e-16, flag, 0));
+    CK(cudaMemcpy(&ok, flag, sizeof(int), cudaMemcpyDeviceToHost));
+    if (!ok) return WM_OK;
+    double* rows = nullptr;
+    const size_t nr = (size_t)B.N[0] * B.N[1] * RT_N;
+    if ((r = c->mem.alloc(&rows, nr))) return r;
+    CK(launch_ext_rows(B.met, B.N, k0, rows, 0));
+    B.rows = rows;
+    B.ktab = d_kt;
+    if (precision == WM_PREC_MIXED) {
+        float *rows32 = nullptr, *kt32 = nullptr;
+        if ((r = c->mem.alloc(&rows32, nr))) return r;
+        if ((r = c->mem.alloc(&kt32, kt.size()))) return r;
+        CK(launch_to_f32(rows, rows32, (long long)nr, 0));
+        CK(launch_to_f32(d_kt, kt32, (long long)kt.size(), 0));
+        B.rows32 = rows32;
+        B.ktab32 = kt32;
+    }
+    return WM_OK;
 }
 
 GhostSeg segment(const wm_case* c, const GhostProg& p, int start, int block0) {
@@ -474,26 +524,15 @@ int build_view(View* v, wm_case* const* cases, int n) {
     int req = cases[0]->chunk_req;
     for (int ci = 1; ci < n; ++ci)
         if (cases[ci]->chunk_req != req) req = 0;
-    int tj, tk;
-    tile_shape(v->opts.tile, &tj, &tk);
-    const int ic = choose_chunk(v->hb, v->opts, tj, tk, req);
-    build_tiles(v, tj, tk, ic);
-    if (req == 0) {
-        // automatic: the wave split when its slowest CTA costs less than the chunked grid's
-        // waves
-        const int slots = stage_slots(v->opts);
-        const long long nt = (long long)v->tiles.size();
-        // a segment's prologue (four planes staged and converted, two gradient planes, one
-        // face plane, with little overlap) charged as 6 planes in this comparison
-        const double chunked = double((nt + slots - 1) / slots) * (ic + 6);
-        View trial;
-        trial.hb = v->hb; trial.nblocks = v->nblocks;
-        if (build_waves(&trial, tj, tk, slots, 6.0) < chunked) {
-            v->tiles = trial.tiles;
-            v->cta_first = trial.cta_first;
-        }
+    for (int b = 0; b < v->nblocks; ++b) v->work[v->hb[b].rows ? 1 : 0].blocks.push_back(b);
+    for (View::Work& w : v->work) {
+        if (w.blocks.empty()) continue;
+        const int ic = choose_chunk(v->hb, w.blocks, v->opts, req);
+        build_tiles(v->hb, &w, ic);
+        if (req != 0) continue;
+        build_waves(v->hb, &w, stage_slots(v->opts));
     }
-    cmf_slots(v, tj, tk);
+    cmf_slots(v);
     v->cta_start.assign(1, 0);                  // one interior cell per thread of the CFL pass
     v->gcta_start.assign(1, 0);                 // one ghost cell per thread
     for (const BlockDev& B : v->hb) {
@@ -505,9 +544,11 @@ int build_view(View* v, wm_case* const* cases, int n) {
     if ((r = m.upload(&v->d_blocks, v->hb.data(), v->hb.size()))) return r;
     if ((r = m.upload(&v->d_cases, v->hc.data(), v->hc.size()))) return r;
     if ((r = m.upload(&v->d_walls, v->hw.data(), v->hw.size()))) return r;
-    if ((r = m.upload(&v->d_tiles, v->tiles.data(), v->tiles.size()))) return r;
-    if (!v->cta_first.empty())
-        if ((r = m.upload(&v->d_cta_first, v->cta_first.data(), v->cta_first.size()))) return r;
+    for (View::Work& w : v->work) {
+        if ((r = m.upload(&w.d_tiles, w.tiles.data(), w.tiles.size()))) return r;
+        if (!w.cta_first.empty())
+            if ((r = m.upload(&w.d_cta_first, w.cta_first.data(), w.cta_first.size()))) return r;
+    }
     if ((r = m.upload(&v->d_case_slot_start, v->case_slot_start.data(), v->case_slot_start.size()))) return r;
     if ((r = m.upload(&v->d_seg_rhs, v->seg_rhs.data(), v->seg_rhs.size()))) return r;
     if ((r = m.upload(&v->d_seg_all, v->seg_all.data(), v->seg_all.size()))) return r;
@@ -580,9 +621,7 @@ int run_stage(View* v, Prof* pf, int stage, double* const* q_in, const double* c
     }
     StageArgs A{};
     A.blocks = v->d_blocks; A.cases = v->d_cases; A.walls = v->d_walls;
-    A.tiles = v->d_tiles; A.ntiles = (int)v->tiles.size();
-    A.cta_first = v->cta_first.empty() ? nullptr : v->d_cta_first;
-    A.nctas = v->cta_first.empty() ? A.ntiles : (int)v->cta_first.size() - 1;
+    A.cmf_ctas = v->work[0].ctas() + v->work[1].ctas();
     A.stage = stage;
     A.ncases = v->ncases;
     A.case_slot_start = v->d_case_slot_start;
@@ -597,8 +636,16 @@ int run_stage(View* v, Prof* pf, int stage, double* const* q_in, const double* c
         A.p[b].spmean = spm[b];
         A.cmf_slot_start[b] = v->cmf_slot_start[b];
     }
-    LaunchScope ls(pf, WM_KIND_STAGE, s);
-    CK(launch_stage(A, v->opts, s));
+    for (int x = 0; x < 2; ++x) {
+        const View::Work& w = v->work[x];
+        if (w.tiles.empty()) continue;
+        A.ext = x;
+        A.tiles = w.d_tiles; A.ntiles = (int)w.tiles.size();
+        A.cta_first = w.d_cta_first;
+        A.nctas = w.ctas();
+        LaunchScope ls(pf, WM_KIND_STAGE, s);
+        CK(launch_stage(A, v->opts, s));
+    }
     return WM_OK;
 }
 
@@ -720,14 +767,15 @@ int wm_case_create(const wm_case_desc* d, wm_case** out) {
         C.sp_sigma0 = d->sponge.strength * d->sponge.U_inf / d->sponge.L;
         C.sp_invL = 1.0 / d->sponge.L;
     }
-    // automatic tile shape: 8x32 for FP64, 16x32 for the mixed form (the fastest on every
-    // measured workload but the C-grid, whose 40-cell k extent the FP64 16x16 tile fits better);
-    // fixed per precision, so cases created with the default can share a batch
-    const int auto_tile = d->precision == WM_PREC_MIXED ? 3 : 0;
-    c->opts = StageOpts{d->precision, d->scheme, d->kep_order, d->limiter, d->sgs, d->tile < 0 ? auto_tile : d->tile};
+    // automatic tile (-1): one kernel variant per precision (so cases created with the default
+    // can share a batch), the tile shape chosen per block from the case's extents alone
+    c->opts = StageOpts{d->precision, d->scheme, d->kep_order, d->limiter, d->sgs, d->tile < 0 ? -1 : d->tile};
 
     // ---- blocks, metrics, work buffers
     c->hb.resize(d->nblocks);
+    const int slots = stage_slots(c->opts);
+    double cells = 0.0;
+    for (int b = 0; b < d->nblocks; ++b) cells += (double)d->blocks[b].n[0] * d->blocks[b].n[1] * d->blocks[b].n[2];
     for (int b = 0; b < d->nblocks; ++b) {
         const wm_block& src = d->blocks[b];
         BlockDev& B = c->hb[b];
@@ -737,6 +785,8 @@ int wm_case_create(const wm_case_desc* d, wm_case** out) {
         B.plane = (long long)B.N[1] * B.N[2];
         B.ncell = B.plane * B.N[0];
         for (int f = 0; f < 6; ++f) B.wall[f] = -1;
+        // each block on its share of the GPU
+        tile_shape(c->opts, B.n, (int)(slots * ((double)B.n[0] * B.n[1] * B.n[2] / cells) + 0.5), &B.tj, &B.tk);
         if (B.ncell * WM_NMET >= (1LL << 31))
             return bail(fail(WM_E_UNSUPPORTED, "block %d: %lld cells exceed the 32-bit metric index range "
                              "(split the block)", b, B.ncell));
@@ -758,6 +808,7 @@ int wm_case_create(const wm_case_desc* d, wm_case** out) {
             CKB(launch_to_f32(met, p32, (long long)nmet, 0));
             B.met32 = p32;
         }
+        if ((r = extruded_tables(c, B, d->precision))) return bail(r);
         for (int s = 0; s < 2; ++s) {
             double* w = nullptr;
             if ((r = c->mem.alloc(&w, 5 * (size_t)B.ncell))) return bail(r);
@@ -1063,9 +1114,10 @@ int wm_batch_info(wm_batch* b, int* nblocks, int* ntiles, long long* launches_pe
     const View& v = b->view;
     int inflow = 0;
     for (wm_case* c : v.members) inflow += c->has_inflow ? 1 : 0;
-    const long long per_stage = IN_LAUNCHES * inflow + ((v.total_rhs || !v.hw.empty() || v.any_sponge) ? 1 : 0) + 1;
+    const long long per_stage = IN_LAUNCHES * inflow + ((v.total_rhs || !v.hw.empty() || v.any_sponge) ? 1 : 0) +
+                                (v.work[0].tiles.empty() ? 0 : 1) + (v.work[1].tiles.empty() ? 0 : 1);
     if (nblocks) *nblocks = v.nblocks;
-    if (ntiles) *ntiles = (int)v.tiles.size();
+    if (ntiles) *ntiles = (int)(v.work[0].tiles.size() + v.work[1].tiles.size());
     if (launches_per_step) *launches_per_step = 3 * per_stage + 1;
     return WM_OK;
 }

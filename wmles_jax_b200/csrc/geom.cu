@@ -14,6 +14,7 @@
 //              the viscous correction geometry e = dx / |dx|, 1 / |dx| with
 //              dx = xc[c] - xc[c - 1] along d and |dx| = sqrt((dx.x^2 + dx.y^2) + dx.z^2),
 //              zero on the first layer (wmles/viscous.py:35-37)
+#include "wm_internal.cuh"
 #include "geom.cuh"
 #include "wmles_cuda.h"
 
@@ -175,7 +176,74 @@ __global__ void __launch_bounds__(GM_NT) to_f32_kernel(const double* __restrict_
         dst[i] = __double2float_rn(src[i]);
 }
 
+__global__ void __launch_bounds__(GM_NT) ext_check_kernel(const double* __restrict__ met, int N0, int N1, int N2, int ng,
+                                                          int k0, const double* __restrict__ ktab, double tol, int* flag) {
+    const long long n = (long long)N0 * N1 * N2;
+    // gradient records one cell beyond the interior, their upper faces one more
+    const int a0 = N0 - 2 * ng + 3, a1 = N1 - 2 * ng + 3, a2 = N2 - 2 * ng + 3;
+    const long long cells = (long long)a0 * a1 * a2;
+    bool ok = true;
+    for (long long t = (long long)blockIdx.x * GM_NT + threadIdx.x; t < cells; t += (long long)gridDim.x * GM_NT) {
+        const int k = ng - 1 + int(t % a2);
+        const long long r = t / a2;
+        const long long row = ((ng - 1 + r / a1) * (long long)N1 + ng - 1 + r % a1) * N2;
+        const double* m = met + row + k;
+        const double* z = met + row + k0;
+        const double rk = ktab[2 * k], idk = ktab[2 * k + 1];
+        auto at = [&](int c) { return m[c * n]; };
+        auto ref = [&](int c) { return z[c * n]; };
+        ok = ok && at(WM_MET_SIZ) == 0.0 && at(WM_MET_SJZ) == 0.0 && at(WM_MET_SKX) == 0.0 && at(WM_MET_SKY) == 0.0 &&
+             at(WM_MET_EIZ) == 0.0 && at(WM_MET_EJZ) == 0.0 && at(WM_MET_EKX) == 0.0 && at(WM_MET_EKY) == 0.0 &&
+             at(WM_MET_EKZ) == 1.0 && fabs(at(WM_MET_SKZ) - ref(WM_MET_SKZ)) <= tol * fabs(ref(WM_MET_SKZ)) &&
+             fabs(at(WM_MET_IDK) - idk) <= tol * idk;
+#pragma unroll
+        for (int d = 0; d < 2; ++d) {
+            const int sx = WM_MET_SIX + 3 * d, ex = WM_MET_EIX + 4 * d;
+            const double s = tol * (fabs(ref(sx)) + fabs(ref(sx + 1)));
+#pragma unroll
+            for (int q = 0; q < 2; ++q)
+                ok = ok && fabs(at(sx + q) - ref(sx + q) * rk) <= s && fabs(at(ex + q) - ref(ex + q)) <= tol;
+            ok = ok && fabs(at(ex + 3) - ref(ex + 3)) <= tol * fabs(ref(ex + 3));
+        }
+    }
+    if (!ok) *flag = 0;
+}
+
+__global__ void __launch_bounds__(GM_NT) ext_rows_kernel(const double* __restrict__ met, int N0, int N1, int N2, int k0,
+                                                         double* __restrict__ rows) {
+    const long long n = (long long)N0 * N1 * N2, nr = (long long)N0 * N1;
+    for (long long r = (long long)blockIdx.x * GM_NT + threadIdx.x; r < nr; r += (long long)gridDim.x * GM_NT) {
+        const double* m = met + r * N2 + k0;
+        const double* u = m + (r / N1 + 1 < N0 ? (long long)N1 * N2 : 0);      // the row of i + 1
+        double* o = rows + r * RT_N;
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            o[RT_SI + q] = m[(WM_MET_SIX + q) * n];
+            o[RT_HI + q] = u[(WM_MET_SIX + q) * n];
+            o[RT_SJ + q] = m[(WM_MET_SJX + q) * n];
+            o[RT_EI + q] = m[(WM_MET_EIX + q) * n];
+            o[RT_EJ + q] = m[(WM_MET_EJX + q) * n];
+        }
+        o[RT_SK] = m[WM_MET_SKZ * n];
+        o[RT_IDI] = m[WM_MET_IDI * n];
+        o[RT_IDJ] = m[WM_MET_IDJ * n];
+        for (int q = RT_IDJ + 1; q < RT_N; ++q) o[q] = 0.0;
+    }
+}
+
 }  // namespace
+
+cudaError_t launch_ext_check(const double* met, const int N[3], int ng, int k0, const double* ktab, double tol, int* flag,
+                             cudaStream_t s) {
+    ext_check_kernel<<<grid_for((long long)N[0] * N[1] * N[2]), GM_NT, 0, s>>>(met, N[0], N[1], N[2], ng, k0, ktab, tol,
+                                                                               flag);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_ext_rows(const double* met, const int N[3], int k0, double* rows, cudaStream_t s) {
+    ext_rows_kernel<<<grid_for((long long)N[0] * N[1]), GM_NT, 0, s>>>(met, N[0], N[1], N[2], k0, rows);
+    return cudaGetLastError();
+}
 
 cudaError_t launch_geometry(const GeomArgs& A, cudaStream_t s) {
     long long maxf = 0;

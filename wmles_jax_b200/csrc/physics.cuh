@@ -22,8 +22,8 @@ struct Phys {
 __device__ __forceinline__ double wm_sqrt(double x) { return sqrt(x); }
 __device__ __forceinline__ float wm_sqrt(float x) { return sqrtf(x); }
 
-// primitive record kept per cell in shared memory: rho, u, v, w, p, T, e = p/((g-1)rho) + |u|^2/2
-enum { PR_RHO = 0, PR_U, PR_V, PR_W, PR_P, PR_T, PR_E, PR_N };
+// primitive record kept per cell in shared memory: rho, u, v, w, p, e = p/((g-1)rho) + |u|^2/2, T
+enum { PR_RHO = 0, PR_U, PR_V, PR_W, PR_P, PR_E, PR_T, PR_N };
 
 // conservative -> primitive record, wmles/gas.py:28-33
 template <typename R>
@@ -45,34 +45,64 @@ __device__ __forceinline__ R sutherland(R T, const Phys<R>& P) {
     return P.mu_ref * (x * wm_sqrt(x)) * P.TrefS / (T + P.S_suth);
 }
 
+// Orientation of a face's area vector S and centre-to-centre vector e, known at compile time on
+// grids extruded along k: FACE_XY (S and e in the x-y plane) leaves out the products with
+// their zero z components, FACE_Z (S = (0, 0, Sz), e = (0, 0, 1)) those with x and y.  The terms
+// left out are exact zeros, so finite results do not change; where the general form adds such a
+// zero to a product, prod() keeps the product rounded by itself in the float form (the same bits
+// as the general form).
+enum { FACE_ANY = 0, FACE_XY = 1, FACE_Z = 2 };
+__device__ __forceinline__ float prod(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double prod(double a, double b) { return a * b; }
+
+// (x, y, z) . S
+template <int FACE, typename R>
+__device__ __forceinline__ R dot_s(R x, R y, R z, R Sx, R Sy, R Sz) {
+    if constexpr (FACE == FACE_XY) return x * Sx + y * Sy;
+    else if constexpr (FACE == FACE_Z) return prod(z, Sz);
+    else return x * Sx + y * Sy + z * Sz;
+}
+// a * b + c * S, where S is the x (A = 0), y or z (A = 2) component.  The float form's contraction is
+// spelled out, or it would be the compiler's choice by what surrounds it and differ by orientation
+template <int FACE, int A>
+__device__ __forceinline__ double madd_s(double a, double b, double c, double S) {
+    if constexpr ((FACE == FACE_XY && A == 2) || (FACE == FACE_Z && A < 2)) return a * b;
+    else return a * b + c * S;
+}
+template <int FACE, int A>
+__device__ __forceinline__ float madd_s(float a, float b, float c, float S) {
+    if constexpr ((FACE == FACE_XY && A == 2) || (FACE == FACE_Z && A < 2)) return __fmul_rn(a, b);
+    else return __fmaf_rn(c, S, __fmul_rn(a, b));
+}
+
 // Kennedy-Gruber two-point flux (already times the face area), wmles/schemes.py:15-23
-template <typename R>
-__device__ __forceinline__ void kg_flux(const R* a, const R* b, int s, R Sx, R Sy, R Sz, R F[5]) {
-    const R rho = R(0.5) * (a[PR_RHO * s] + b[PR_RHO * s]);
-    const R u = R(0.5) * (a[PR_U * s] + b[PR_U * s]);
-    const R v = R(0.5) * (a[PR_V * s] + b[PR_V * s]);
-    const R w = R(0.5) * (a[PR_W * s] + b[PR_W * s]);
-    const R p = R(0.5) * (a[PR_P * s] + b[PR_P * s]);
-    const R ea = R(0.5) * (a[PR_E * s] + b[PR_E * s]);
-    const R un = u * Sx + v * Sy + w * Sz;
+template <int FACE, typename R>
+__device__ __forceinline__ void kg_flux(const R* a, int sa, const R* b, int s, R Sx, R Sy, R Sz, R F[5]) {
+    const R rho = R(0.5) * (a[PR_RHO * sa] + b[PR_RHO * s]);
+    const R u = R(0.5) * (a[PR_U * sa] + b[PR_U * s]);
+    const R v = R(0.5) * (a[PR_V * sa] + b[PR_V * s]);
+    const R w = R(0.5) * (a[PR_W * sa] + b[PR_W * s]);
+    const R p = R(0.5) * (a[PR_P * sa] + b[PR_P * s]);
+    const R ea = R(0.5) * (a[PR_E * sa] + b[PR_E * s]);
+    const R un = dot_s<FACE>(u, v, w, Sx, Sy, Sz);
     const R m = rho * un;
     F[0] = m;
-    F[1] = m * u + p * Sx;
-    F[2] = m * v + p * Sy;
-    F[3] = m * w + p * Sz;
+    F[1] = madd_s<FACE, 0>(m, u, p, Sx);
+    F[2] = madd_s<FACE, 1>(m, v, p, Sy);
+    F[3] = madd_s<FACE, 2>(m, w, p, Sz);
     F[4] = m * ea + p * un;
 }
 
 // KEP order 2 / 4, wmles/schemes.py:57-70: 2 [(2/3) F(L,R) - (1/12) (F(L,R2) + F(L2,R))],
 // written (4/3) F(L,R) - (1/6) (...) (the outer factor 2 moved into the constants: exact)
-template <typename R>
-__device__ __forceinline__ void kep_flux(int order, const R* L2, const R* L, const R* Rr, const R* R2,
-                                         int s, R Sx, R Sy, R Sz, R F[5]) {
-    kg_flux(L, Rr, s, Sx, Sy, Sz, F);
+template <int FACE, typename R>
+__device__ __forceinline__ void kep_flux(int order, const R* L2, int s2, const R* L, const R* Rr,
+                                         const R* R2, int s, R Sx, R Sy, R Sz, R F[5]) {
+    kg_flux<FACE>(L, s, Rr, s, Sx, Sy, Sz, F);
     if (order == 4) {
         R Fa[5], Fb[5];
-        kg_flux(L, R2, s, Sx, Sy, Sz, Fa);
-        kg_flux(L2, Rr, s, Sx, Sy, Sz, Fb);
+        kg_flux<FACE>(L, s, R2, s, Sx, Sy, Sz, Fa);
+        kg_flux<FACE>(L2, s2, Rr, s, Sx, Sy, Sz, Fb);
 #pragma unroll
         for (int v = 0; v < 5; ++v)
             F[v] = R(4.0 / 3.0) * F[v] - R(1.0 / 6.0) * (Fa[v] + Fb[v]);
@@ -92,18 +122,40 @@ __device__ __forceinline__ R minmod(R a, R b) {
     return R(0.5) * (sgn(a) + sgn(b)) * fmin(fabs(a), fabs(b));
 }
 
-// HLLC flux times |S|, wmles/schemes.py:108-137
+// both limited slopes of one variable at a face, albada(a, b) and albada(b, c).  FP64: the two
+// quotients from one division (1 / (d1 d2) times the other denominator; the denominators are at
+// least 2e-12), as a division is some 30 instructions and a face takes ten
 template <typename R>
+__device__ __forceinline__ void albada2(R a, R b, R c, R& l, R& r) {
+    if constexpr (sizeof(R) == 8) {
+        const R eps = R(1e-12);
+        const R a2 = a * a, b2 = b * b, c2 = c * c;
+        const R d1 = a2 + b2 + R(2) * eps, d2 = b2 + c2 + R(2) * eps;
+        const R q = R(1) / (d1 * d2);
+        l = (a * (b2 + eps) + b * (a2 + eps)) * (d2 * q);
+        r = (b * (c2 + eps) + c * (b2 + eps)) * (d1 * q);
+    } else {
+        l = albada(a, b);
+        r = albada(b, c);
+    }
+}
+
+// HLLC flux times |S|, wmles/schemes.py:108-137
+template <int FACE, typename R>
 __device__ __forceinline__ void hllc_flux(const R wl[5], const R wr[5], R Sx, R Sy, R Sz, R gamma,
                                           R inv_gm1, R F[5]) {
-    const R Sm = wm_sqrt(Sx * Sx + Sy * Sy + Sz * Sz);
+    const R Sm = wm_sqrt(dot_s<FACE>(Sx, Sy, Sz, Sx, Sy, Sz));
     const R iS = R(1) / Sm;
     const R nx = Sx * iS, ny = Sy * iS, nz = Sz * iS;
+    constexpr bool D = sizeof(R) == 8;           // FP64: quotients that share a division (below)
     const R rl = wl[0], ul = wl[1], vl = wl[2], wlz = wl[3], pl = wl[4];
     const R rr = wr[0], ur = wr[1], vr = wr[2], wrz = wr[3], pr = wr[4];
-    const R unl = ul * nx + vl * ny + wlz * nz;
-    const R unr = ur * nx + vr * ny + wrz * nz;
-    const R cl = wm_sqrt(gamma * pl / rl), cr = wm_sqrt(gamma * pr / rr);
+    const R unl = dot_s<FACE>(ul, vl, wlz, nx, ny, nz);
+    const R unr = dot_s<FACE>(ur, vr, wrz, nx, ny, nz);
+    // FP64: 1 / rl and 1 / rr from 1 / (rl rr), later 1 / (s - un) and 1 / (s - ss) from their
+    // product's: four divisions a face instead of seven, of some 30 instructions each
+    const R irr = D ? R(1) / (rl * rr) : R(0), il = rr * irr, ir = rl * irr;
+    const R cl = wm_sqrt(D ? gamma * pl * il : gamma * pl / rl), cr = wm_sqrt(D ? gamma * pr * ir : gamma * pr / rr);
     const R sL = fmin(unl - cl, unr - cr), sR = fmax(unl + cl, unr + cr);
     const R ss = (pr - pl + rl * unl * (sL - unl) - rr * unr * (sR - unr)) /
                  (rl * (sL - unl) - rr * (sR - unr));
@@ -114,20 +166,28 @@ __device__ __forceinline__ void hllc_flux(const R wl[5], const R wr[5], R Sx, R 
     const R E = p * inv_gm1 + R(0.5) * r * (u * u + v * v + w * w);
     R Fp[5];
     Fp[0] = r * un;
-    Fp[1] = r * un * u + p * nx;
-    Fp[2] = r * un * v + p * ny;
-    Fp[3] = r * un * w + p * nz;
+    Fp[1] = madd_s<FACE, 0>(r * un, u, p, nx);
+    Fp[2] = madd_s<FACE, 1>(r * un, v, p, ny);
+    Fp[3] = madd_s<FACE, 2>(r * un, w, p, nz);
     Fp[4] = (E + p) * un;
     const bool star = left ? !(sL >= R(0)) : (sR > R(0));
     if (star) {
         const R s = left ? sL : sR;
-        const R f = r * (s - un) / (s - ss);
-        const R e = E / r + (ss - un) * (ss + p / (r * (s - un)));
+        R f, e;
+        if constexpr (D) {
+            const R q = R(1) / ((s - un) * (s - ss));
+            const R iro = left ? il : ir;
+            f = r * (s - un) * ((s - un) * q);
+            e = E * iro + (ss - un) * (ss + p * iro * ((s - ss) * q));
+        } else {
+            f = r * (s - un) / (s - ss);
+            e = E / r + (ss - un) * (ss + p / (r * (s - un)));
+        }
         const R d = ss - un;
         Fp[0] += s * (f - r);
-        Fp[1] += s * (f * (u + d * nx) - r * u);
-        Fp[2] += s * (f * (v + d * ny) - r * v);
-        Fp[3] += s * (f * (w + d * nz) - r * w);
+        Fp[1] += s * (f * (FACE == FACE_Z ? u : u + d * nx) - r * u);
+        Fp[2] += s * (f * (FACE == FACE_Z ? v : v + d * ny) - r * v);
+        Fp[3] += s * (f * (FACE == FACE_XY ? w : w + d * nz) - r * w);
         Fp[4] += s * (f * e - E);
     }
 #pragma unroll
@@ -135,27 +195,29 @@ __device__ __forceinline__ void hllc_flux(const R wl[5], const R wr[5], R Sx, R 
 }
 
 // MUSCL reconstruction with positivity fallback + HLLC, wmles/schemes.py:140-152
-template <typename R>
-__device__ __forceinline__ void muscl_hllc_flux(int limiter, const R* L2, const R* L, const R* Rr,
+template <int FACE, typename R>
+__device__ __forceinline__ void muscl_hllc_flux(int limiter, const R* L2, int s2, const R* L, const R* Rr,
                                                 const R* R2, int s, R Sx, R Sy, R Sz,
                                                 const Phys<R>& P, R F[5]) {
     R wl[5], wr[5];
 #pragma unroll
     for (int v = 0; v < 5; ++v) {
-        const R a = L[v * s] - L2[v * s], b = Rr[v * s] - L[v * s], c = R2[v * s] - Rr[v * s];
+        const R a = L[v * s] - L2[v * s2], b = Rr[v * s] - L[v * s], c = R2[v * s] - Rr[v * s];
         if (limiter == WM_LIMITER_MINMOD) {
             wl[v] = L[v * s] + R(0.5) * minmod(a, b);
             wr[v] = Rr[v * s] - R(0.5) * minmod(b, c);
         } else {
-            wl[v] = L[v * s] + R(0.5) * albada(a, b);
-            wr[v] = Rr[v * s] - R(0.5) * albada(b, c);
+            R sl, sr;
+            albada2(a, b, c, sl, sr);
+            wl[v] = L[v * s] + R(0.5) * sl;
+            wr[v] = Rr[v * s] - R(0.5) * sr;
         }
     }
     if (wl[0] <= R(0) || wl[4] <= R(0) || wr[0] <= R(0) || wr[4] <= R(0)) {
 #pragma unroll
         for (int v = 0; v < 5; ++v) { wl[v] = L[v * s]; wr[v] = Rr[v * s]; }
     }
-    hllc_flux(wl, wr, Sx, Sy, Sz, P.gamma, P.inv_gm1, F);
+    hllc_flux<FACE>(wl, wr, Sx, Sy, Sz, P.gamma, P.inv_gm1, F);
 }
 
 // SGS eddy viscosity nu_t from g[i][j] = du_i/dx_j, wmles/sgs.py:14-42

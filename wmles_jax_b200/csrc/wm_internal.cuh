@@ -39,7 +39,16 @@ struct BlockDev {
     const double* met;     // WM_NMET x ncell (float64)
     const float* met32;    // WM_NMET x ncell (float32 copy for the mixed form), may be null
     int wall[6];       // view wall index of face (axis*2 + side), -1 if not wall-modelled
+    int tj, tk;        // shape of its stage tiles
+    // blocks extruded along k (ext_check in geom.cu): metrics per (i, j) row and per k; else null
+    const double* rows;    // N[0] x N[1] x RT_N
+    const double* ktab;    // N[2] x 2: area factor of i and j faces, inverse centre distance to k - 1
+    const float *rows32, *ktab32;   // rounded copies (mixed form)
 };
+
+// entries of a row of an extruded block (x, y components unless noted)
+enum { RT_SI = 0, RT_HI = 2 /* lower, upper i face */, RT_SJ = 4, RT_SK = 6 /* z */, RT_EI = 7, RT_IDI = 9,
+       RT_EJ = 10, RT_IDJ = 12, RT_N = 16 };
 
 // per-case physical constants, precomputed where the kernels only need a derived value
 struct CaseDev {
@@ -69,6 +78,8 @@ struct WallDev {
 // stage-kernel work item: one (j,k) tile of one block over planes [i0, i1)
 struct Tile {
     int blk, j0, k0, i0, i1;   // blk: view block index
+    int tj, tk;                // extents of this tile (the block's last ones may be smaller)
+    int col;                   // index of its (j,k) column in the block
 };
 
 // one case's ghost-cell program inside a view-wide gather launch
@@ -109,6 +120,8 @@ struct StageArgs {
     const int* case_slot_start;   // ncases + 1: partial-sum slots of case c are [start[c], start[c+1])
     double* cmf_part;             // stage 3 with constant mass flux: per (column, plane, warp) partials
     unsigned int* cmf_counter;    // last-CTA-done counter (the last CTA resets it)
+    int cmf_ctas;                 // CTAs of the stage's launches
+    int ext;                      // the tiles' blocks are extruded along k
     double* cmf_delta;            // per case: constant-mass-flux shift, written by the last CTA
     const double* dt[MAX_CASES];  // per case: device time step
     int cmf_slot_start[WM_MAX_BLOCKS];   // first partial-sum slot of each block
