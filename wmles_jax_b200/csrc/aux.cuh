@@ -42,6 +42,7 @@ struct DtArgs {
     const double* cmf_delta;       // per case: constant-mass-flux shift from stage 3 (null: none)
     int want_dt;                   // 0: constraint only
     int met32;                     // read the float metric copy (mixed form)
+    int ext;                       // every block is extruded along k
     unsigned long long* dt_key;    // per case: running minimum as an order-preserving key
                                    // (DT_KEY_EMPTY between calls: reset by the last CTA)
     unsigned int* counter;         // last-CTA-done counter (reset by the last CTA)

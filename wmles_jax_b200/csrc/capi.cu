@@ -442,11 +442,10 @@ int extruded_tables(wm_case* c, BlockDev& B, int precision) {
         kt[2 * k + 1] = id[k];
         if (!(kt[2 * k] > 0.0)) return WM_OK;
     }
-    Owner tmp;
     double* d_kt = nullptr;
     int *flag = nullptr, ok = 1;
     int r;
-    if ((r = tmp.upload(&flag, &ok, 1))) return r;
+    if ((r = c->mem.upload(&flag, &ok, 1))) return r;      // kept: a cudaFree here would wait for the device
     if ((r = c->mem.upload(&d_kt, kt.data(), kt.size()))) return r;
     CK(launch_ext_check(B.met, B.N, B.ng, k0, d_kt, 16 * 2.220446049250313e-16, flag, 0));
     CK(cudaMemcpy(&ok, flag, sizeof(int), cudaMemcpyDeviceToHost));
@@ -666,6 +665,7 @@ int run_dt(View* v, Prof* pf, double* const* q, bool apply_cmf, bool want_dt, do
     D.cmf_delta = apply_cmf ? v->cmf_delta : nullptr;
     D.want_dt = want_dt ? 1 : 0;
     D.met32 = v->opts.precision == WM_PREC_MIXED ? 1 : 0;
+    D.ext = v->work[0].blocks.empty() ? 1 : 0;
     D.dt_key = v->dt_key; D.counter = v->counters;
     for (int ci = 0; ci < v->ncases; ++ci) D.dt_out[ci] = dt_out ? dt_out[ci] : nullptr;
     LaunchScope ls(pf, WM_KIND_DT, s);
@@ -756,6 +756,7 @@ int wm_case_create(const wm_case_desc* d, wm_case** out) {
     C.sgs_c = d->sgs_coeff;
     C.cfl = d->cfl;
     C.nu_fac = std::max(4.0 / 3.0, g.gamma / g.Pr);
+    C.c_ref = std::sqrt(g.gamma * g.R * g.T_ref);
     C.Pr13 = std::pow(g.Pr, 1.0 / 3.0);
     C.Pr3 = std::pow(g.Pr, 3.0);
     C.kader_beta = std::pow(3.85 * std::pow(g.Pr, 1.0 / 3.0) - 1.3, 2.0) + 2.12 * std::log(g.Pr);
@@ -785,6 +786,8 @@ int wm_case_create(const wm_case_desc* d, wm_case** out) {
         B.plane = (long long)B.N[1] * B.N[2];
         B.ncell = B.plane * B.N[0];
         for (int f = 0; f < 6; ++f) B.wall[f] = -1;
+        B.div_nj.set(B.n[1]);
+        B.div_nk.set(B.n[2]);
         // each block on its share of the GPU
         tile_shape(c->opts, B.n, (int)(slots * ((double)B.n[0] * B.n[1] * B.n[2] / cells) + 0.5), &B.tj, &B.tk);
         if (B.ncell * WM_NMET >= (1LL << 31))

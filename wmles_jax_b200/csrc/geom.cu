@@ -227,7 +227,18 @@ __global__ void __launch_bounds__(GM_NT) ext_rows_kernel(const double* __restric
         o[RT_SK] = m[WM_MET_SKZ * n];
         o[RT_IDI] = m[WM_MET_IDI * n];
         o[RT_IDJ] = m[WM_MET_IDJ * n];
-        for (int q = RT_IDJ + 1; q < RT_N; ++q) o[q] = 0.0;
+        const double* w = m + (r % N1 + 1 < N1 ? N2 : 0);                          // the row of j + 1
+        double len[2];
+#pragma unroll
+        for (int d = 0; d < 2; ++d) {
+            const double* h = d == 0 ? u : w;
+            const int sx = WM_MET_SIX + 3 * d;
+            const double x = 0.5 * (m[sx * n] + h[sx * n]), y = 0.5 * (m[(sx + 1) * n] + h[(sx + 1) * n]);
+            len[d] = sqrt(x * x + y * y);
+        }
+        o[RT_MI] = len[0];
+        o[RT_MJ] = len[1];
+        for (int q = RT_MJ + 1; q < RT_N; ++q) o[q] = 0.0;
     }
 }
 

@@ -107,17 +107,6 @@ __device__ __forceinline__ const R* metbase(const BlockDev& B) {
     if constexpr (sizeof(R) == 4) return B.met32;
     else return B.met;
 }
-template <typename R>
-__device__ __forceinline__ const R* rows_of(const BlockDev& B) {
-    if constexpr (sizeof(R) == 4) return B.rows32;
-    else return B.rows;
-}
-template <typename R>
-__device__ __forceinline__ const R* ktab_of(const BlockDev& B) {
-    if constexpr (sizeof(R) == 4) return B.ktab32;
-    else return B.ktab;
-}
-
 __device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
     const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem) : "memory");

@@ -28,6 +28,20 @@ inline cudaError_t once_per_device(std::atomic<unsigned long long>& done, F set)
 
 constexpr int MAX_CASES = WM_MAX_BLOCKS;   // a case has at least one block
 
+// x / d of a divisor known at set-up, for 0 <= x < 2^31: (x mul) >> shift with mul = ceil(2^shift / d),
+// shift = 31 + ceil(log2 d) (mul < 2^33 x 2^31 fits 64 bits; exact for 31-bit x)
+struct FastDiv {
+    unsigned long long mul;
+    int shift;
+    __host__ void set(unsigned d) {
+        int l = 0;
+        while ((1u << l) < d) ++l;
+        shift = 31 + l;
+        mul = ((1ull << shift) + d - 1) / d;
+    }
+    __host__ __device__ int operator()(unsigned x) const { return (int)((x * mul) >> shift); }
+};
+
 // one structured block, resident in device memory
 struct BlockDev {
     int n[3];          // interior cells
@@ -40,6 +54,7 @@ struct BlockDev {
     const float* met32;    // WM_NMET x ncell (float32 copy for the mixed form), may be null
     int wall[6];       // view wall index of face (axis*2 + side), -1 if not wall-modelled
     int tj, tk;        // shape of its stage tiles
+    FastDiv div_nj, div_nk;   // by n[1], n[2]
     // blocks extruded along k (ext_check in geom.cu): metrics per (i, j) row and per k; else null
     const double* rows;    // N[0] x N[1] x RT_N
     const double* ktab;    // N[2] x 2: area factor of i and j faces, inverse centre distance to k - 1
@@ -48,7 +63,19 @@ struct BlockDev {
 
 // entries of a row of an extruded block (x, y components unless noted)
 enum { RT_SI = 0, RT_HI = 2 /* lower, upper i face */, RT_SJ = 4, RT_SK = 6 /* z */, RT_EI = 7, RT_IDI = 9,
-       RT_EJ = 10, RT_IDJ = 12, RT_N = 16 };
+       RT_EJ = 10, RT_IDJ = 12,
+       RT_MI = 13, RT_MJ = 14 /* lengths of the means of the lower and upper i and j face vectors */, RT_N = 16 };
+
+template <typename R>
+__device__ __forceinline__ const R* rows_of(const BlockDev& B) {
+    if constexpr (sizeof(R) == 4) return B.rows32;
+    else return B.rows;
+}
+template <typename R>
+__device__ __forceinline__ const R* ktab_of(const BlockDev& B) {
+    if constexpr (sizeof(R) == 4) return B.ktab32;
+    else return B.ktab;
+}
 
 // per-case physical constants, precomputed where the kernels only need a derived value
 struct CaseDev {
@@ -57,6 +84,7 @@ struct CaseDev {
     double th0, inv_dth;   // Hybrid: s = clip((theta - th0) * inv_dth, 0, 1)
     double sgs_c;          // model coefficient
     double cfl, nu_fac;    // nu_fac = max(4/3, gamma/Pr)
+    double c_ref;          // speed of sound at T_ref
     double Pr13, Pr3, kader_beta;   // Pr^(1/3), Pr^3, (3.85 Pr^(1/3) - 1.3)^2 + 2.12 ln Pr
     int cmf_dir;
     double cmf_target, cmf_volume;
