@@ -911,8 +911,8 @@ int wm_case_create(const wm_case_desc* d, wm_case** out) {
     int max_nj = 1;
     for (const BlockDev& B : c->hb) max_nj = std::max(max_nj, B.n[1]);
     if ((r = c->mem.alloc(&c->ps_part, (size_t)PS_NQ * max_nj * PS_CHUNKS))) return bail(r);
-    if ((r = c->mem.alloc(&c->ps_counter, 1))) return bail(r);
-    CKB(cudaMemset(c->ps_counter, 0, sizeof(unsigned)));
+    if ((r = c->mem.alloc(&c->ps_counter, (size_t)max_nj))) return bail(r);
+    CKB(cudaMemset(c->ps_counter, 0, sizeof(unsigned) * max_nj));
 
     // ---- status word (every view of the case points at it)
     if ((r = c->mem.alloc(&c->d_status, 1))) return bail(r);
@@ -1029,7 +1029,7 @@ int wm_plane_stats(wm_case* c, int block, const double* q, double* sum, void* st
     A.q = q;
     A.gm1 = c->hc.gm1;
     A.Rg = c->hc.Rg;
-    A.nchunks = PS_CHUNKS;
+    A.nchunks = plane_chunks(c->hb[block].n[0], c->hb[block].n[1]);
     A.part = c->ps_part;
     A.sum = sum;
     A.counter = c->ps_counter;
@@ -1049,8 +1049,7 @@ int wm_derived_fields(wm_case* c, const double* const* q, double* const* out, vo
         A.sgs = c->opts.sgs;
         A.q = q[b];
         A.out = out[b];
-        const BlockDev& B = v->hb[b];
-        CK(launch_derived(A, (long long)B.n[0] * B.n[1] * B.n[2], (cudaStream_t)stream));
+        CK(launch_derived(A, v->hb[b].n, (cudaStream_t)stream));
     }
     return WM_OK;
 }

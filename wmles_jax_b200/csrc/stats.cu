@@ -5,39 +5,64 @@
 //
 // One CTA per (i-chunk, plane): each thread walks its cells of the chunk and keeps the 12
 // FP64 sums in registers; a block reduction writes one partial per quantity; the last CTA of
-// the launch adds, per plane and quantity, the chunk partials in chunk order divided by the
-// plane's cell count (a fixed order: the result does not depend on scheduling).
+// a plane adds, per quantity, the plane's chunk partials in chunk order divided by its cell count (a
+// fixed order: the result does not depend on scheduling).
+//
+// What bounds it: the state is read once (40 B per cell), so HBM if enough loads are in flight
+// and the arithmetic is short: one reciprocal per cell instead of four divisions, two cells
+// per thread at a time, as many chunks as one wave of CTAs holds (plane_chunks), and a last CTA
+// per plane (one for all planes took 11 us by itself).  192 x 96 x 96: 59 -> 23 us.
+#include <algorithm>
 #include <cfloat>
 #include "wm_internal.cuh"
 #include "stats.cuh"
 
 namespace wm {
 
-constexpr int PS_NT = 256;
+constexpr int PS_NT = 128, PS_CPS = 8;       // threads per CTA, CTAs resident per SM
 
-__global__ void __launch_bounds__(PS_NT) plane_stats_kernel(const __grid_constant__ PlaneStatsArgs A) {
+__global__ void __launch_bounds__(PS_NT, PS_CPS) plane_stats_kernel(const __grid_constant__ PlaneStatsArgs A) {
     __shared__ double red[PS_NQ][PS_NT / 32];
     __shared__ bool last;
     const BlockDev& B = *A.block;
-    const int ng = B.ng, ni = B.n[0], nk = B.n[2], Nj = B.N[1], Nk = B.N[2];
+    const int ng = B.ng, ni = B.n[0], nk = B.n[2], Nk = B.N[2], plane = (int)B.plane;
     const int chunk = blockIdx.x, jj = blockIdx.y;          // jj: interior plane index
     const int i0 = (int)((long long)chunk * ni / A.nchunks), i1 = (int)((long long)(chunk + 1) * ni / A.nchunks);
     const long long N = B.ncell;
+    const FastDiv div_nk = B.div_nk;
+    const double* q = A.q;
+    const double iRg = 1.0 / A.Rg;
     double acc[PS_NQ];
 #pragma unroll
-    for (int q = 0; q < PS_NQ; ++q) acc[q] = 0.0;
-    const int cells = (i1 - i0) * nk;
-    for (int c = threadIdx.x; c < cells; c += PS_NT) {
-        const int i = i0 + c / nk + ng, k = c % nk + ng;
-        const long long idx = ((long long)i * Nj + (jj + ng)) * Nk + k;
-        // gas.cons_to_prim (wmles/gas.py:28-33)
-        const double rho = A.q[idx];
-        const double u = A.q[N + idx] / rho, v = A.q[2 * N + idx] / rho, w = A.q[3 * N + idx] / rho;
-        const double p = A.gm1 * (A.q[4 * N + idx] - (0.5 * rho) * ((u * u + v * v) + w * w));
-        const double T = p / (rho * A.Rg);
-        const double x[PS_NQ] = {rho, u, v, w, u * u, v * v, w * w, u * v, u * w, v * w, T, p};
+    for (int x = 0; x < PS_NQ; ++x) acc[x] = 0.0;
+    const int cells = (i1 - i0) * nk, base = (i0 + ng) * plane + (jj + ng) * Nk + ng;
+    auto load = [&](int c, double w[5]) {
+        const int i = div_nk(c);
+        const int idx = base + i * plane + (c - i * nk);
 #pragma unroll
-        for (int q = 0; q < PS_NQ; ++q) acc[q] += x[q];
+        for (int v = 0; v < 5; ++v) w[v] = __ldg(q + v * N + idx);
+    };
+    auto add = [&](const double w[5]) {
+        // gas.cons_to_prim (wmles/gas.py:28-33)
+        const double rho = w[0], ir = 1.0 / rho;
+        const double u = w[1] * ir, v = w[2] * ir, ww = w[3] * ir;
+        const double p = A.gm1 * (w[4] - (0.5 * rho) * ((u * u + v * v) + ww * ww));
+        const double x[PS_NQ] = {rho, u, v, ww, u * u, v * v, ww * ww, u * v, u * ww, v * ww, p * ir * iRg, p};
+#pragma unroll
+        for (int y = 0; y < PS_NQ; ++y) acc[y] += x[y];
+    };
+    int c = threadIdx.x;
+    for (; c + PS_NT < cells; c += 2 * PS_NT) {
+        double wa[5], wb[5];
+        load(c, wa);
+        load(c + PS_NT, wb);
+        add(wa);
+        add(wb);
+    }
+    if (c < cells) {
+        double wa[5];
+        load(c, wa);
+        add(wa);
     }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
@@ -55,18 +80,24 @@ __global__ void __launch_bounds__(PS_NT) plane_stats_kernel(const __grid_constan
         __threadfence();
     }
     __syncthreads();
-    if (threadIdx.x == 0) last = atomicAdd(A.counter, 1u) == gridDim.x * gridDim.y - 1;
+    if (threadIdx.x == 0) last = atomicAdd(A.counter + jj, 1u) == gridDim.x - 1;
     __syncthreads();
     if (!last) return;
     __threadfence();
-    const volatile double* part = A.part;
-    const double inv = 1.0 / ((double)ni * nk);
-    for (int e = threadIdx.x; e < PS_NQ * B.n[1]; e += PS_NT) {
+    if (threadIdx.x < PS_NQ) {
+        const long long e = (long long)threadIdx.x * B.n[1] + jj;
         double s = 0.0;
-        for (int ch = 0; ch < A.nchunks; ++ch) s += part[(long long)e * A.nchunks + ch];
-        A.sum[e] += s * inv;
+#pragma unroll 8
+        for (int ch = 0; ch < A.nchunks; ++ch) s += __ldcg(A.part + e * A.nchunks + ch);
+        A.sum[e] += s * (1.0 / ((double)ni * nk));
     }
-    if (threadIdx.x == 0) *A.counter = 0u;
+    if (threadIdx.x == 0) A.counter[jj] = 0u;
+}
+
+// chunks per plane: one wave of CTAs on 148 SMs (a constant, so that the order of the sums does
+// not depend on the device), at most PS_CHUNKS and one plane of cells each
+int plane_chunks(int ni, int nj) {
+    return std::max(1, std::min({PS_CHUNKS, ni, 148 * PS_CPS / std::max(1, nj)}));
 }
 
 cudaError_t launch_plane_stats(const PlaneStatsArgs& A, int nj, cudaStream_t s) {

@@ -22,7 +22,7 @@ def derived_fields(solver, Q, time=0.0, as_numpy=True):
     result = {}
     for ib, o in enumerate(outs):
         f = dict(zip(NAMES, o))
-        d = {"rho": f["rho"], "velocity": torch.stack([f["u"], f["v"], f["w"]]), "pressure": f["pressure"],
+        d = {"rho": f["rho"], "velocity": o[1:4], "pressure": f["pressure"],
              "temperature": f["temperature"], "mach": f["mach"], "mu_t": f["mu_t"], "mu": f["mu"],
              "vorticity_mag": f["vorticity_mag"], "q_criterion": f["q_criterion"]}
         result[ib] = {k: v.cpu().numpy() for k, v in d.items()} if as_numpy else d
