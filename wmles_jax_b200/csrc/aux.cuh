@@ -132,7 +132,7 @@ struct SurfaceArgs {
     GhostArgs G;
     WallArgs W;
     SpongeArgs S;          // nblocks = 0: no sponge
-    int g_ctas, w_per, w_ctas, s_ctas;
+    int g_ctas, w_nt, w_per, w_ctas, s_ctas;     // w_nt: wall faces per CTA, w_per: CTAs per wall
 };
 
 __device__ __forceinline__ long long cell_index(const BlockDev& B, int axis, int c, int a, int b) {

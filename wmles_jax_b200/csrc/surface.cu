@@ -13,6 +13,7 @@
 // Before every stage kernel one launch (surface_kernel) does all three: the parts read
 // disjoint data (ghost cells are written; the wall model and the sponge means read interior
 // cells only), so they overlap instead of running as three dependent launches.
+#include <algorithm>
 #include "wm_internal.cuh"
 #include "physics.cuh"
 #include "aux.cuh"
@@ -312,7 +313,7 @@ __global__ void __launch_bounds__(SURF_NT, 4) surface_kernel(const __grid_consta
     int bx = blockIdx.x;
     if (bx < A.w_ctas) {
         const int w = bx / A.w_per;
-        wall_face(A.W, w, (long long)(bx - w * A.w_per) * SURF_NT + threadIdx.x);
+        if ((int)threadIdx.x < A.w_nt) wall_face(A.W, w, (long long)(bx - w * A.w_per) * A.w_nt + threadIdx.x);
         return;
     }
     bx -= A.w_ctas;
@@ -328,7 +329,13 @@ __global__ void __launch_bounds__(SURF_NT, 4) surface_kernel(const __grid_consta
 
 cudaError_t launch_surface(SurfaceArgs& A, cudaStream_t s) {
     A.g_ctas = (A.G.total + SURF_NT - 1) / SURF_NT;
-    A.w_per = A.W.nwalls ? (A.W.max_faces + SURF_NT - 1) / SURF_NT : 0;
+    // wall faces per CTA: as few as spread them over the chip (148 SMs; a face is a chain of FP64 operations
+    // and the warps of one SM share its FP64 units), in whole warps, at most one per thread.  Channel
+    // 32 x 32 x 16 (1024 faces, 32 per CTA instead of 256), with the Newton iteration's start and stop:
+    // 12.4 -> 9.2 us a launch
+    const int spread = (A.W.nwalls * A.W.max_faces / 148 + 31) / 32 * 32;
+    A.w_nt = std::max(32, std::min(SURF_NT, spread));
+    A.w_per = A.W.nwalls ? (A.W.max_faces + A.w_nt - 1) / A.w_nt : 0;
     A.w_ctas = A.w_per * A.W.nwalls;
     A.s_ctas = (A.S.nrows + SURF_NT / 32 - 1) / (SURF_NT / 32);
     const int n = A.g_ctas + A.w_ctas + A.s_ctas;
