@@ -45,6 +45,24 @@ __device__ __forceinline__ double dt_value_of(unsigned long long k) {
     return __longlong_as_double((long long)((k >> 63) ? (k & 0x7fffffffffffffffull) : ~k));
 }
 
+// the constant-mass-flux shift of momentum component m (1..3) and energy; selects instead of qv[m], so
+// that the state stays in registers
+__device__ __forceinline__ void cmf_shift(double qv[5], int m, double delta) {
+    const double qm = m == 1 ? qv[1] : m == 2 ? qv[2] : qv[3];
+    const double dE = (2.0 * qm * delta + delta * delta) / (2.0 * qv[0]), qn = qm + delta;
+#pragma unroll
+    for (int v = 1; v < 4; ++v) qv[v] = v == m ? qn : qv[v];
+    qv[4] = qv[4] + dE;
+}
+
+// a descriptor into shared memory, by the CTA's threads together
+template <typename T>
+__device__ __forceinline__ void copy_words(T* dst, const T* src) {
+    static_assert(sizeof(T) % 8 == 0 && alignof(T) == 8, "copied as 64-bit words");
+    for (int w = threadIdx.x; w < int(sizeof(T) / 8); w += blockDim.x)
+        reinterpret_cast<unsigned long long*>(dst)[w] = reinterpret_cast<const unsigned long long*>(src)[w];
+}
+
 // CFL time step (Solver._dt, wmles/solver.py:135-151), optionally after applying the
 // constant-mass-flux shift (ConstantMassFlux.__call__, wmles/solver.py:22-36) in place.
 // The view's interior cells are cut into chunks of DT_NT cells, one cell per thread, chunks
@@ -92,10 +110,8 @@ __global__ void __launch_bounds__(DT_NT, EXT || sizeof(M) == 4 ? 4 : 3) dt_kerne
             }
             bend = D.cta_start[b + 1];
             __syncthreads();
-            if (threadIdx.x == 0) {
-                B = D.blocks[b];
-                C = D.cases[B.case_id];
-            }
+            copy_words(&B, D.blocks + b);
+            copy_words(&C, D.cases + D.blocks[b].case_id);
             __syncthreads();
             if (D.want_dt && B.case_id != cur) {
                 if (cur >= 0) flush();
@@ -155,10 +171,8 @@ __global__ void __launch_bounds__(DT_NT, EXT || sizeof(M) == 4 ? 4 : 3) dt_kerne
             if (cmf) {
                 const double delta = D.cmf_delta[B.case_id];
                 const int m = 1 + C.cmf_dir;
-                const double dE = (2.0 * qv[m] * delta + delta * delta) / (2.0 * qv[0]);
-                qv[m] = qv[m] + delta;
-                qv[4] = qv[4] + dE;
-                q[m * N + idx] = qv[m];
+                cmf_shift(qv, m, delta);
+                q[m * N + idx] = m == 1 ? qv[1] : m == 2 ? qv[2] : qv[3];
                 q[4 * N + idx] = qv[4];
             }
             const double rho = qv[0];
@@ -239,9 +253,7 @@ __global__ void __launch_bounds__(DT_NT, EXT || sizeof(M) == 4 ? 4 : 3) dt_kerne
                 // the reference shifts every cell, ghost cells included (wmles/solver.py:30-36)
                 const double delta = D.cmf_delta[B.case_id];
                 const int m = 1 + C.cmf_dir;
-                const double dE = (2.0 * qv[m] * delta + delta * delta) / (2.0 * qv[0]);
-                qv[m] = qv[m] + delta;
-                qv[4] = qv[4] + dE;
+                cmf_shift(qv, m, delta);
             }
 #pragma unroll
             for (int v = 0; v < 5; ++v) q[v * N + idx] = qv[v];
