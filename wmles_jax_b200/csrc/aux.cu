@@ -76,6 +76,7 @@ __device__ __forceinline__ void copy_words(T* dst, const T* src) {
 // in the other instance, without the registers of the general form).
 template <typename M, bool EXT>
 __global__ void __launch_bounds__(DT_NT, EXT || sizeof(M) == 4 ? 4 : 3) dt_kernel(const __grid_constant__ DtArgs D) {
+    chain_wait();
     __shared__ bool last;
     double run = DBL_MAX;          // this thread's minimum over its cells of case `cur`
     int cur = -1;
@@ -307,15 +308,14 @@ static int dt_wave() {
 }
 
 template <typename M, bool EXT>
-static void launch_dt_one(const DtArgs& D, cudaStream_t s) {
+static cudaError_t launch_dt_one(const DtArgs& D, cudaStream_t s) {
     const int chunks = std::max(D.ncta, D.ngcta);
-    dt_kernel<M, EXT><<<std::max(1, std::min(chunks, dt_wave<M, EXT>())), DT_NT, 0, s>>>(D);
+    return launch_chained(dt_kernel<M, EXT>, std::max(1, std::min(chunks, dt_wave<M, EXT>())), DT_NT, 0, s, D);
 }
 
 cudaError_t launch_dt(const DtArgs& D, cudaStream_t s) {
-    if (D.met32) D.ext ? launch_dt_one<float, true>(D, s) : launch_dt_one<float, false>(D, s);
-    else D.ext ? launch_dt_one<double, true>(D, s) : launch_dt_one<double, false>(D, s);
-    return cudaGetLastError();
+    if (D.met32) return D.ext ? launch_dt_one<float, true>(D, s) : launch_dt_one<float, false>(D, s);
+    return D.ext ? launch_dt_one<double, true>(D, s) : launch_dt_one<double, false>(D, s);
 }
 
 // ------------------------------------------------------------------ synthetic inflow

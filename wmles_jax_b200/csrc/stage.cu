@@ -111,6 +111,13 @@ __device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
     const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem) : "memory");
 }
+// a value of a state: not by the read-only path, which wants data that nothing writes during the kernel's
+// life, and this kernel may come up while the launch before it still writes (chain_wait)
+__device__ __forceinline__ double ld_state(const double* p) {
+    double v;
+    asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
+    return v;
+}
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p)); }
 __device__ __forceinline__ void prefetch_l1(const void* p) { asm volatile("prefetch.global.L1 [%0];\n" ::"l"(p)); }
@@ -565,10 +572,10 @@ __device__ __forceinline__ void stage_segment(const StageArgs& A, const StageOpt
         const int idx = io * planei + ct[c];
         e.ivol = __ldg(MB + WM_MET_IVOL * nc + idx);
 #pragma unroll
-        for (int v = 0; v < 5; ++v) e.q[v] = __ldg(SP.q_in + v * nc + idx);
+        for (int v = 0; v < 5; ++v) e.q[v] = ld_state(SP.q_in + v * nc + idx);
         if (A.stage >= 2) {
 #pragma unroll
-            for (int v = 0; v < 5; ++v) e.q0[v] = __ldg(SP.q0 + v * nc + idx);
+            for (int v = 0; v < 5; ++v) e.q0[v] = ld_state(SP.q0 + v * nc + idx);
         }
         if (cmf_on) e.vol = __ldg(B.met + WM_MET_VOL * nc + idx);
     };
@@ -638,7 +645,7 @@ __device__ __forceinline__ void stage_segment(const StageArgs& A, const StageOpt
 #pragma unroll
         for (int d = 0; d < PRE; ++d)
 #pragma unroll
-            for (int v = 0; v < 5; ++v) q[d][v] = __ldg(src + d * planei + v * nc);
+            for (int v = 0; v < 5; ++v) q[d][v] = ld_state(src + d * planei + v * nc);
 #pragma unroll
         for (int d = 0; d < PRE; ++d) {
             R rec[PR_N];
@@ -695,7 +702,7 @@ __device__ __forceinline__ void stage_segment(const StageArgs& A, const StageOpt
                 const bool ok = c < npr && ip + 3 <= i1 + 1;
                 const double* src = SP.q_in + (ok ? (ip + 3) * planei + pt[c] : 0);
 #pragma unroll
-                for (int v = 0; v < 5; ++v) cq[r][v] = ok ? __ldg(src + v * nc) : 0.0;
+                for (int v = 0; v < 5; ++v) cq[r][v] = ok ? ld_state(src + v * nc) : 0.0;
             }
 #pragma unroll
             for (int r = 0; r < 2; ++r) {
@@ -705,8 +712,8 @@ __device__ __forceinline__ void stage_segment(const StageArgs& A, const StageOpt
                 e[r].ivol = ok ? __ldg(MB + WM_MET_IVOL * nc + idx) : R(0);
 #pragma unroll
                 for (int v = 0; v < 5; ++v) {
-                    e[r].q[v] = ok ? __ldg(SP.q_in + v * nc + idx) : 0.0;
-                    e[r].q0[v] = ok && A.stage >= 2 ? __ldg(SP.q0 + v * nc + idx) : 0.0;
+                    e[r].q[v] = ok ? ld_state(SP.q_in + v * nc + idx) : 0.0;
+                    e[r].q0[v] = ok && A.stage >= 2 ? ld_state(SP.q0 + v * nc + idx) : 0.0;
                 }
                 e[r].vol = ok && cmf_on ? __ldg(B.met + WM_MET_VOL * nc + idx) : 0.0;
             }
@@ -848,6 +855,7 @@ template <typename R, int SCHEME, int CAP, bool EXT>
 __global__ void __launch_bounds__(StageLayout<R, SCHEME, CAP, EXT>::NTH, StageLayout<R, SCHEME, CAP, EXT>::MIN_CTAS)
     stage_kernel(const __grid_constant__ StageArgs A, const StageOpts o) {
     using LY = StageLayout<R, SCHEME, CAP, EXT>;
+    chain_wait();
     constexpr int NTH = LY::NTH;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double* red = reinterpret_cast<double*>(smem_raw + LY::red_off);
@@ -911,8 +919,7 @@ static cudaError_t launch_one(const StageArgs& A, const StageOpts& o, cudaStream
     using LY = StageLayout<R, SCHEME, CAP, EXT>;
     cudaError_t e = configure_one<R, SCHEME, CAP, EXT>();
     if (e != cudaSuccess) return e;
-    stage_kernel<R, SCHEME, CAP, EXT><<<A.nctas, LY::NTH, LY::bytes, s>>>(A, o);
-    return cudaGetLastError();
+    return launch_chained(stage_kernel<R, SCHEME, CAP, EXT>, A.nctas, LY::NTH, LY::bytes, s, A, o);
 }
 
 template <typename R, int SCHEME, int CAP, bool EXT>

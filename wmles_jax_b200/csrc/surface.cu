@@ -310,6 +310,7 @@ constexpr int SURF_NT = 256;
 // SM (64 registers, a few spills in the wall part) rather than three at 80: the ghost entries
 // are chains of dependent loads and gain from the extra warps (channel surface time -7 %).
 __global__ void __launch_bounds__(SURF_NT, 4) surface_kernel(const __grid_constant__ SurfaceArgs A) {
+    chain_wait();
     int bx = blockIdx.x;
     if (bx < A.w_ctas) {
         const int w = bx / A.w_per;
@@ -340,8 +341,7 @@ cudaError_t launch_surface(SurfaceArgs& A, cudaStream_t s) {
     A.s_ctas = (A.S.nrows + SURF_NT / 32 - 1) / (SURF_NT / 32);
     const int n = A.g_ctas + A.w_ctas + A.s_ctas;
     if (n == 0) return cudaSuccess;
-    surface_kernel<<<n, SURF_NT, 0, s>>>(A);
-    return cudaGetLastError();
+    return launch_chained(surface_kernel, n, SURF_NT, 0, s, A);
 }
 
 }  // namespace wm
