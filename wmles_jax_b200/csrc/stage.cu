@@ -60,7 +60,14 @@ struct StageLayout {
     static constexpr int FN = stage_caps(CAP).fn;      // j faces, then k faces
     static constexpr int RN = EXT ? stage_caps(CAP).rows : 0;      // rows of the tile + 1-row halo + 1
     static constexpr int KN = EXT ? stage_caps(CAP).kn : 0;        // k positions of the tile + 1-cell halo
-    static constexpr int NGS = (SCHEME == WM_SCHEME_HYBRID) ? 15 : 14;
+    // values of a gradient record, and how many of them lie side by side: component v of record c at
+    // [v / GV][c][v % GV], so that a face takes a record in 16-byte loads.  General grids, where these
+    // loads wait in one queue with those of the metrics: fours (float) or pairs (FP64; the Hybrid form has
+    // no room for the 16th value).  Box 160 x 96 x 72, KEP, float 1117 -> 1083 us for two steps, box 75 x
+    // 53 x 37, MUSCL, FP64 485 -> 472.  Extruded grids have fewer loads and, in float, no registers
+    // to spare: channel, three steps, float 3681 -> 3945, FP64 6411 -> 6461, so one by one there
+    static constexpr int GV = EXT ? 1 : sizeof(R) == 4 ? 4 : SCHEME == WM_SCHEME_HYBRID ? 1 : 2;
+    static constexpr int NGS = GV == 4 ? 16 : (SCHEME == WM_SCHEME_HYBRID) ? 15 : 14;
     // FP64, one CTA per SM: a fifth primitive slot (the shared memory is there), so plane
     // i+2 is converted while the gradient records of plane i are computed, by the warps that
     // have no record to compute, and a plane takes two barriers instead of three.  The float
@@ -94,6 +101,7 @@ struct StageLayout {
     static constexpr int GW = (GN + 31) / 32 * 32;     // threads of the warps with a record, at most
     static_assert(!FUSE || 2 * (NTH - GW) >= CAP, "at most two epilogue columns per thread");
     static_assert(rt_off % 16 == 0, "rows arrive in 16-byte pieces");
+    static_assert(GV == 1 || gs_off % 16 == 0, "gradient records are read in 16-byte pieces");
     static_assert(bytes * MIN_CTAS <= 227 * 1024, "shared memory of an SM");
 };
 
@@ -136,13 +144,26 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
 template <int FACE, typename R, class GL, class GR>
 __device__ __forceinline__ void viscous_flux(const R* pl, const R* pr, int s, GL gL, GR gR, R Sx, R Sy, R Sz,
                                              R e0, R e1, R e2, R idist, R V[4]) {
-    R gf[12];
+    // a record's components one by one, or GW at a time (StageLayout::GW)
+    constexpr int GW = sizeof(decltype(gL(0))) / sizeof(R);
+    R gf[12], sum[GW > 1 ? 16 : 1];
+    if constexpr (GW > 1) {
+#pragma unroll
+        for (int x = 0; x < (GS_TH + GW - 1) / GW; ++x) {
+            const auto l = gL(x), r = gR(x);
+#pragma unroll
+            for (int y = 0; y < GW; ++y)
+                sum[GW * x + y] = reinterpret_cast<const R*>(&l)[y] + reinterpret_cast<const R*>(&r)[y];
+        }
+    }
+    auto add = [&](int v) {
+        if constexpr (GW > 1) return sum[v];
+        else return gL(v) + gR(v);
+    };
     const int pv[4] = {PR_U, PR_V, PR_W, PR_T};
 #pragma unroll
     for (int a = 0; a < 4; ++a) {
-        const R b0 = gL(3 * a) + gR(3 * a);
-        const R b1 = gL(3 * a + 1) + gR(3 * a + 1);
-        const R b2 = gL(3 * a + 2) + gR(3 * a + 2);
+        const R b0 = add(3 * a), b1 = add(3 * a + 1), b2 = add(3 * a + 2);
         const R be = FACE == FACE_Z ? b2 : FACE == FACE_XY ? b0 * e0 + b1 * e1 : b0 * e0 + b1 * e1 + b2 * e2;
         const R corr = (pr[pv[a] * s] - pl[pv[a] * s]) * idist - be;
         gf[3 * a] = FACE == FACE_Z ? b0 : b0 + corr * e0;
@@ -150,8 +171,8 @@ __device__ __forceinline__ void viscous_flux(const R* pl, const R* pr, int s, GL
         gf[3 * a + 2] = FACE == FACE_Z ? b2 + corr : FACE == FACE_XY ? b2 : b2 + corr * e2;
     }
     const R div = gf[0] + gf[4] + gf[8];
-    const R muf = gL(GS_MU) + gR(GS_MU);
-    const R kf = gL(GS_K) + gR(GS_K);
+    const R muf = add(GS_MU);
+    const R kf = add(GS_K);
     const R d23 = R(2.0 / 3.0) * div;
     const R t00 = muf * (gf[0] + gf[0] - d23), t11 = muf * (gf[4] + gf[4] - d23), t22 = muf * (gf[8] + gf[8] - d23);
     const R t01 = muf * (gf[1] + gf[3]), t02 = muf * (gf[2] + gf[6]), t12 = muf * (gf[5] + gf[7]);
@@ -212,7 +233,10 @@ __device__ __forceinline__ void face_flux(const StageOpts& o, const Phys<R>& P, 
             muscl_flux<FACE>(o.limiter, P, L2, s2, L, Rr, R2, s, Sx, Sy, Sz, F);
         } else {
             // Ducros-switched blend, wmles/schemes.py:163-166
-            const R th = fmax(gL(GS_TH), gR(GS_TH));
+            R th;
+            constexpr int GW = sizeof(decltype(gL(0))) / sizeof(R);
+            if constexpr (GW == 4) th = fmax(gL(3).z, gR(3).z);
+            else th = fmax(gL(GS_TH), gR(GS_TH));
             const R sw = fmin(fmax((th - P.th0) * P.inv_dth, R(0)), R(1));
             R Fc[5] = {R(0), R(0), R(0), R(0), R(0)}, Fu[5] = {R(0), R(0), R(0), R(0), R(0)};
             if (sw > R(0)) muscl_flux<FACE>(o.limiter, P, L2, s2, L, Rr, R2, s, Sx, Sy, Sz, Fu);
@@ -317,6 +341,8 @@ __device__ __forceinline__ void stage_segment(const StageArgs& A, const StageOpt
         }
     }
 
+    using GV = std::conditional_t<LY::GV == 1, R, std::conditional_t<LY::GV == 2, double2, float4>>;
+    constexpr int NGV = NGS / LY::GV;
     // ring slot of plane ip + d; `ring` is the slot of the march's plane, stepped with it
     constexpr int SLOT = PR_N * PN, RING = LY::NSLOT * SLOT;
     int ring = 0;
@@ -426,11 +452,26 @@ __device__ __forceinline__ void stage_segment(const StageArgs& A, const StageOpt
             const R rho = P0[PR_RHO * PN + pc];
             muth = rho * sgs_nut(sgs_model, acc, delta, P.sgs_c);
         }
+        const R mu = muh + muth, kc = P.cp * (muh * P.inv_Pr + muth * P.inv_Prt);
+        R th = R(0);
+        if constexpr (SCHEME == WM_SCHEME_HYBRID) th = ducros(acc);
+        if constexpr (LY::GV == 1) {
 #pragma unroll
-        for (int q = 0; q < 12; ++q) gs[q * GN + c] = acc[q];
-        gs[GS_MU * GN + c] = muh + muth;
-        gs[GS_K * GN + c] = P.cp * (muh * P.inv_Pr + muth * P.inv_Prt);
-        if constexpr (NGS > 14) gs[GS_TH * GN + c] = ducros(acc);
+            for (int q = 0; q < 12; ++q) gs[q * GN + c] = acc[q];
+            gs[GS_MU * GN + c] = mu;
+            gs[GS_K * GN + c] = kc;
+            if constexpr (NGS > 14) gs[GS_TH * GN + c] = th;
+        } else {
+            R rec[16] = {acc[0], acc[1], acc[2], acc[3], acc[4], acc[5], acc[6], acc[7], acc[8], acc[9], acc[10], acc[11], mu, kc, th, R(0)};
+            GV* g = reinterpret_cast<GV*>(gs) + c;
+#pragma unroll
+            for (int x = 0; x < NGV; ++x) {
+                GV y;
+#pragma unroll
+                for (int w = 0; w < LY::GV; ++w) reinterpret_cast<R*>(&y)[w] = rec[LY::GV * x + w];
+                g[x * GN] = y;
+            }
+        }
     };
 
     // wall-model flux override of a wall-modelled face (axis, side) at its position (a, b); EXT, i and j
@@ -445,13 +486,19 @@ __device__ __forceinline__ void stage_segment(const StageArgs& A, const StageOpt
     };
 
     // ---- i-face flux between planes ip-1 and ip for this thread's column
-    R gsp[FUSE ? 1 : NGS];   // float form: gradient record of plane ip-1 at this column
+    // float form: gradient record of plane ip-1 at this column
+    GV gsp[FUSE ? 1 : NGV];
     auto save_gs = [&]() {
         if constexpr (!FUSE) {
             if (!column) return;
 #pragma unroll
-            for (int v = 0; v < NGS; ++v) gsp[v] = gs[v * GN + col_gc];
+            for (int v = 0; v < NGV; ++v) gsp[v] = reinterpret_cast<const GV*>(gs)[v * GN + col_gc];
         }
+    };
+    // record c + off of the march's plane: its components or, GV > 1, groups of them
+    auto grad_at = [&](int c, int off) {
+        const GV* g = reinterpret_cast<const GV*>(gs) + c;
+        return [g, off](int v) { return g[v * GN + off]; };
     };
     auto iface_flux = [&](int ip, R F[5]) {
         if ((ip == ng && iwall0) || (ip == ihi && iwall1)) {
@@ -464,9 +511,13 @@ __device__ __forceinline__ void stage_segment(const StageArgs& A, const StageOpt
         const R* L = slot(-1) + col_pc;
         const R* Rr = slot(0) + col_pc;
         const R* R2 = slot(1) + col_pc;
-        const R* gl = LY::PING ? gs0 + (gs == gs0 ? NGS * GN : 0) + col_gc : hg;
-        auto gL = [&](int v) { return FUSE ? gl[v * (LY::PING ? GN : CAP)] : gsp[FUSE ? 0 : v]; };
-        auto gR = [&](int v) { return gs[v * GN + col_gc]; };
+        const GV* gl = LY::PING ? reinterpret_cast<const GV*>(gs0 + (gs == gs0 ? NGS * GN : 0)) + col_gc
+                                : reinterpret_cast<const GV*>(hg);
+        auto gL = [&](int v) {
+            if constexpr (FUSE) return gl[v * (LY::PING ? GN : CAP)];
+            else return gsp[v];
+        };
+        auto gR = grad_at(col_gc, 0);
         if constexpr (EXT) {
             const R* row = rt + (ip & 1) * LY::RN * RT_N + (tj + 1) * RT_N;
             face_flux<FACE_XY, R, SCHEME>(o, P, L2, S2, L, Rr, R2, PN, gL, gR, row[RT_SI], row[RT_SI + 1], R(0), row[RT_EI],
@@ -491,16 +542,16 @@ __device__ __forceinline__ void stage_segment(const StageArgs& A, const StageOpt
         } else {
             const int pc = (row + 2) * PK + col + 2;
             const R* p = slot(0) + pc;
-            const R* g = gs + (row + 1) * GK + col + 1;
-            auto gR = [&](int v) { return g[v * GN]; };
+            const int gc = (row + 1) * GK + col + 1;
+            auto gR = grad_at(gc, 0);
             if constexpr (EXT) {
                 const R* mr = rt + (ip & 1) * LY::RN * RT_N + (row + 1) * RT_N;
                 if (kf) {
-                    face_flux<FACE_Z, R, SCHEME>(o, P, p - 2, PN, p - 1, p, p + 1, PN, [&](int v) { return g[v * GN - 1]; }, gR,
+                    face_flux<FACE_Z, R, SCHEME>(o, P, p - 2, PN, p - 1, p, p + 1, PN, grad_at(gc, -1), gR,
                                                  R(0), R(0), mr[RT_SK], R(0), R(0), R(1), kt[2 * col + 3], F);
                 } else {
                     face_flux<FACE_XY, R, SCHEME>(o, P, p - 2 * PK, PN, p - PK, p, p + PK, PN,
-                                                  [&](int v) { return g[v * GN - GK]; }, gR, mr[RT_SJ], mr[RT_SJ + 1],
+                                                  grad_at(gc, -GK), gR, mr[RT_SJ], mr[RT_SJ + 1],
                                                   R(0), mr[RT_EJ], mr[RT_EJ + 1], R(0), mr[RT_IDJ], F);
                 }
             } else {
@@ -510,7 +561,7 @@ __device__ __forceinline__ void stage_segment(const StageArgs& A, const StageOpt
                 m += (kf ? WM_MET_EKX - WM_MET_SKX : WM_MET_EJX - WM_MET_SJX) * nc;
                 const R e0 = __ldg(m), e1 = __ldg(m + nc), e2 = __ldg(m + 2 * nc), id = __ldg(m + 3 * nc);
                 face_flux<FACE_ANY, R, SCHEME>(o, P, p - 2 * ps, PN, p - ps, p, p + ps, PN,
-                                               [&](int v) { return g[v * GN - gp]; }, gR, Sx, Sy, Sz, e0, e1, e2, id, F);
+                                               grad_at(gc, -gp), gR, Sx, Sy, Sz, e0, e1, e2, id, F);
             }
         }
 #pragma unroll
@@ -779,7 +830,7 @@ __device__ __forceinline__ void stage_segment(const StageArgs& A, const StageOpt
                 const R* L = slot(-1) + col_pc;
 #pragma unroll
                 for (int v = 0; v < LY::HP_N; ++v) hp[v * CAP] = L[v * PN];
-                if constexpr (!LY::PING) {
+                if constexpr (!LY::PING) {   // EXT: components one by one
 #pragma unroll
                     for (int v = 0; v < NGS; ++v) hg[v * CAP] = gs[v * GN + col_gc];
                 }
