@@ -63,6 +63,24 @@ __device__ __forceinline__ void copy_words(T* dst, const T* src) {
         reinterpret_cast<unsigned long long*>(dst)[w] = reinterpret_cast<const unsigned long long*>(src)[w];
 }
 
+// a case's constants of the CFL rate in its precision, converted once per block (by every cell: channel
+// 256 x 128 x 128, float form, 86 us against 82)
+template <typename M>
+struct DtPhys {
+    M gRg, inv_Rg, inv_Tref, nu_fac, mu_ref, TrefS, S_suth, cfl, c_ref;
+    __device__ __forceinline__ void set(const CaseDev& C) {
+        gRg = M(C.gamma) * M(C.Rg);
+        inv_Rg = M(C.inv_Rg);
+        inv_Tref = M(C.inv_Tref);
+        nu_fac = M(C.nu_fac);
+        mu_ref = M(C.mu_ref);
+        TrefS = M(C.TrefS);
+        S_suth = M(C.S_suth);
+        cfl = M(C.cfl);
+        c_ref = M(C.c_ref);
+    }
+};
+
 // CFL time step (Solver._dt, wmles/solver.py:135-151), optionally after applying the
 // constant-mass-flux shift (ConstantMassFlux.__call__, wmles/solver.py:22-36) in place.
 // The view's interior cells are cut into chunks of DT_NT cells, one cell per thread, chunks
@@ -78,6 +96,7 @@ template <typename M, bool EXT>
 __global__ void __launch_bounds__(DT_NT, EXT || sizeof(M) == 4 ? 4 : 3) dt_kernel(const __grid_constant__ DtArgs D) {
     chain_wait();
     __shared__ bool last;
+    __shared__ DtPhys<M> P;
     double run = DBL_MAX;          // this thread's minimum over its cells of case `cur`
     int cur = -1;
     auto flush = [&]() {
@@ -110,14 +129,16 @@ __global__ void __launch_bounds__(DT_NT, EXT || sizeof(M) == 4 ? 4 : 3) dt_kerne
                 if (D.cta_start[mid] <= chunk) b = mid; else hi = mid - 1;
             }
             bend = D.cta_start[b + 1];
+            const int ci = D.blocks[b].case_id;
+            if (D.want_dt && ci != cur) {
+                if (cur >= 0) flush();
+                cur = ci;
+            }
             __syncthreads();
             copy_words(&B, D.blocks + b);
-            copy_words(&C, D.cases + D.blocks[b].case_id);
+            copy_words(&C, D.cases + ci);
+            if (threadIdx.x == 0) P.set(D.cases[ci]);
             __syncthreads();
-            if (D.want_dt && B.case_id != cur) {
-                if (cur >= 0) flush();
-                cur = B.case_id;
-            }
         }
         const bool cmf = D.cmf_delta != nullptr && C.cmf_dir >= 0;
         const unsigned c = (unsigned)(chunk - D.cta_start[b]) * DT_NT + threadIdx.x;   // cells fit 31 bits
@@ -196,14 +217,14 @@ __global__ void __launch_bounds__(DT_NT, EXT || sizeof(M) == 4 ? 4 : 3) dt_kerne
                 // sqrt(T / T_ref), and cfl V / (lam + 4 nu S2 / V) is cfl / (iv (lam + 4 nu S2 iv)).
                 // Channel 256 x 128 x 128, with the rows' areas and the descriptors in shared memory: 134 ->
                 // 91 us a pass (float form 110 -> 92, its rate unchanged)
-                const double iv = vol, T = p * ir * C.inv_Rg, x = T * C.inv_Tref, rx = sqrt(x);
-                const double nu = C.nu_fac * (C.mu_ref * (x * rx) * C.TrefS / (T + C.S_suth)) * ir;
+                const double iv = vol, T = p * ir * P.inv_Rg, x = T * P.inv_Tref, rx = sqrt(x);
+                const double nu = P.nu_fac * (P.mu_ref * (x * rx) * P.TrefS / (T + P.S_suth)) * ir;
                 const double sk = fabs(Sl[8]);
                 const double lam = (fabs(u * (0.5 * (Sl[0] + Sh[0])) + v * (0.5 * (Sl[1] + Sh[1]))) +
                                     fabs(u * (0.5 * (Sl[3] + Sh[3])) + v * (0.5 * (Sl[4] + Sh[4])))) +
-                                   fabs(w) * sk + C.c_ref * rx * ((mi + mj) + sk);
+                                   fabs(w) * sk + P.c_ref * rx * ((mi + mj) + sk);
                 const double s2 = (mi * mi + mj * mj) + sk * sk;
-                run = nanmin(run, C.cfl / (iv * (lam + 4.0 * nu * s2 * iv)));
+                run = nanmin(run, P.cfl / (iv * (lam + 4.0 * nu * s2 * iv)));
             } else if (D.want_dt) {
                 // the cell's CFL rate in the metric precision: FP64 in the FP64 form; FP32 in the
                 // mixed form, from its FP32 metric copy like its fluxes (the state, its checks,
@@ -211,10 +232,10 @@ __global__ void __launch_bounds__(DT_NT, EXT || sizeof(M) == 4 ? 4 : 3) dt_kerne
                 using CF = M;
                 const CF ivol = CF(1) / vol;
                 const CF irc = CF(ir);
-                const CF T = CF(p) * irc * CF(C.inv_Rg);
-                const CF cs = sqrt(CF(C.gamma) * CF(C.Rg) * T);
-                const CF x = T * CF(C.inv_Tref);
-                const CF nu = CF(C.nu_fac) * (CF(C.mu_ref) * (x * sqrt(x)) * CF(C.TrefS) / (T + CF(C.S_suth))) * irc;
+                const CF T = CF(p) * irc * P.inv_Rg;
+                const CF cs = sqrt(P.gRg * T);
+                const CF x = T * P.inv_Tref;
+                const CF nu = P.nu_fac * (P.mu_ref * (x * sqrt(x)) * P.TrefS / (T + P.S_suth)) * irc;
                 const CF uc = CF(u), vc = CF(v), wc = CF(w);
                 CF lam = CF(0), lamv = CF(0);
 #pragma unroll
@@ -226,7 +247,7 @@ __global__ void __launch_bounds__(DT_NT, EXT || sizeof(M) == 4 ? 4 : 3) dt_kerne
                     lam = lam + fabs((uc * sx + vc * sy) + wc * sz) + cs * Sm;
                     lamv = lamv + nu * (Sm * Sm) * ivol;
                 }
-                run = nanmin(run, double(CF(C.cfl) * vol / (lam + CF(4) * lamv)));
+                run = nanmin(run, double(P.cfl * vol / (lam + CF(4) * lamv)));
             }
         }
     }
@@ -241,10 +262,11 @@ __global__ void __launch_bounds__(DT_NT, EXT || sizeof(M) == 4 ? 4 : 3) dt_kerne
             }
         }
         const BlockDev& B = D.blocks[b];
-        const long long g = (long long)(chunk - D.gcta_start[b]) * DT_NT + threadIdx.x;
-        if (g < ghost_cells(B)) {
+        const unsigned g = (unsigned)(chunk - D.gcta_start[b]) * DT_NT + threadIdx.x;
+        if (g < (unsigned)ghost_cells(B)) {
             const CaseDev& C = D.cases[B.case_id];
-            const long long N = B.ncell, idx = ghost_cell_index(B, g);
+            const long long N = B.ncell;
+            const int idx = ghost_cell_index(B, g);
             const double* src = D.q_src[b];
             double* q = D.q[b];
             double qv[5];

@@ -57,30 +57,20 @@ __host__ __device__ inline long long ghost_cells(const BlockDev& B) {
 // flat index of ghost cell g (0 <= g < ghost_cells(B)), enumerated as the ghost planes
 // i < ng, i >= ng + ni (all j, k), then for interior i the ghost rows in j (all k), then for
 // interior (i, j) the ghost cells in k
-__device__ __forceinline__ long long ghost_cell_index(const BlockDev& B, long long g) {
-    const int ng = B.ng, ni = B.n[0], nj = B.n[1], nk = B.n[2], Nj = B.N[1], Nk = B.N[2];
-    const long long a = 2LL * ng * Nj * Nk;
-    if (g < a) {
-        const int p = int(g / ((long long)Nj * Nk));
-        const long long r = g - (long long)p * Nj * Nk;
-        const int i = p < ng ? p : ni + p;
-        return (long long)i * Nj * Nk + r;
-    }
+__device__ __forceinline__ int ghost_cell_index(const BlockDev& B, unsigned g) {     // cells fit 31 bits
+    const unsigned ng = B.ng, ni = B.n[0], nj = B.n[1], nk = B.n[2], Nj = B.N[1], Nk = B.N[2];
+    const unsigned plane = Nj * Nk, a = 2 * ng * plane;
+    if (g < a) return int(g < ng * plane ? g : ni * plane + g);
     g -= a;
-    const long long b = (long long)ni * 2 * ng * Nk;
+    const unsigned strip = 2 * ng * Nk, b = ni * strip;
     if (g < b) {
-        const int ii = int(g / (2LL * ng * Nk));
-        const int r = int(g - (long long)ii * 2 * ng * Nk);
-        const int p = r / Nk, k = r - p * Nk;
-        const int j = p < ng ? p : nj + p;
-        return ((long long)(ng + ii) * Nj + j) * Nk + k;
+        const unsigned ii = g / strip, r = g - ii * strip;
+        return int((ng + ii) * plane + (r < ng * Nk ? r : nj * Nk + r));
     }
     g -= b;
-    const long long t = g / (2 * ng);
-    const int p = int(g - t * 2 * ng);
-    const int ii = int(t / nj), jj = int(t - (long long)ii * nj);
-    const int k = p < ng ? p : nk + p;
-    return ((long long)(ng + ii) * Nj + (ng + jj)) * Nk + k;
+    const unsigned t = g / (2 * ng), p = g - t * 2 * ng;
+    const unsigned ii = B.div_nj(t), jj = t - ii * nj;
+    return int((ng + ii) * plane + (ng + jj) * Nk + (p < ng ? p : nk + p));
 }
 
 // key of DBL_MAX, the value of an empty minimum (the reset value of DtArgs::dt_key)
