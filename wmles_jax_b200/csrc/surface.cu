@@ -108,11 +108,14 @@ __device__ __forceinline__ int find_seg(const GhostArgs& G, int e) {
 }
 
 // ghost entry e of the launch: gather its source value and apply its map chain; the value
-// goes to the destination ghost cell, or to the stash in two-phase mode
+// goes to the destination ghost cell, or to the stash in two-phase mode.  An entry is a chain of
+// dependent loads, so all its table values are loaded at once, the destination too (looked up
+// after the maps: channel surface launch 24.8 us instead of 23.1; two entries a thread: 26.8)
 __device__ __forceinline__ void ghost_entry(const GhostArgs& G, int e) {
     const GhostSeg& S = G.segs[find_seg(G, e)];
     const int le = e - S.start;
-    const int sk = S.src[2 * le], sc = S.src[2 * le + 1];
+    const int sk = S.src[2 * le], sc = S.src[2 * le + 1], db = S.block0 + S.dst[2 * le], dc = S.dst[2 * le + 1];
+    const int o0 = S.ops[2 * le], no = S.ops[2 * le + 1];
     const int kind = sk >> 24, sb = sk & 0xffffff;
     double q[5];
     if (kind == WM_SRC_CELL) {
@@ -127,7 +130,6 @@ __device__ __forceinline__ void ghost_entry(const GhostArgs& G, int e) {
 #pragma unroll
         for (int v = 0; v < 5; ++v) q[v] = S.bc[8 * sb + v];
     }
-    const int o0 = S.ops[2 * le], no = S.ops[2 * le + 1];
     for (int i = 0; i < no; ++i) {
         const int code = S.op_code[o0 + i];
         const double* nrm = S.op_nrm + 3 * (o0 + i);
@@ -139,7 +141,6 @@ __device__ __forceinline__ void ghost_entry(const GhostArgs& G, int e) {
             default: break;
         }
     }
-    const int db = S.block0 + S.dst[2 * le], dc = S.dst[2 * le + 1];
     if (G.stash != nullptr) {
         // two-phase mode: values first, scatter after every source has been read
 #pragma unroll
