@@ -135,10 +135,13 @@ def check(status, what):
 
 def ptr_array(ptrs):
     """(double*)[] from integer device addresses."""
-    arr = (c_double_p * len(ptrs))()
-    for i, p in enumerate(ptrs):
-        arr[i] = C.cast(C.c_void_p(int(p)), c_double_p)
-    return arr
+    n = len(ptrs)
+    return (c_double_p * n).from_buffer((C.c_void_p * n)(*map(int, ptrs)))
+
+
+def ptr(p):
+    """double* from an integer device address."""
+    return C.cast(int(p), c_double_p)
 
 
 def as_int_p(a):

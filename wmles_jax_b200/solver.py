@@ -226,7 +226,8 @@ class Solver:
         return N.ptr_array([q.data_ptr() for q in Q])
 
     def _stream(self):
-        return C.c_void_p(torch.cuda.current_stream(self.device).cuda_stream)
+        # the handle alone (the device has its index, require_gpu): torch.cuda.current_stream builds a Stream
+        return C.c_void_p(torch._C._cuda_getCurrentRawStream(self.device.index))
 
     def _dt_tensor(self, dt):
         if isinstance(dt, torch.Tensor):
@@ -265,7 +266,7 @@ class Solver:
         """CFL time step as a 0-d CUDA tensor (``float(dt)`` synchronises)."""
         self._check_state(Q)
         dt = torch.empty((), dtype=torch.float64, device=self.device)
-        N.check(self._lib.wm_max_dt(self._case, self._ptrs(Q), N.ptr_array([dt.data_ptr()])[0], self._stream()),
+        N.check(self._lib.wm_max_dt(self._case, self._ptrs(Q), N.ptr(dt.data_ptr()), self._stream()),
                 "wm_max_dt")
         return dt
 
@@ -278,7 +279,7 @@ class Solver:
         self._check_state(Q)
         dtt = self._dt_tensor(dt)
         out = tuple(torch.empty_like(q) for q in Q)
-        N.check(self._lib.wm_advance(self._case, self._ptrs(Q), self._ptrs(out), N.ptr_array([dtt.data_ptr()])[0],
+        N.check(self._lib.wm_advance(self._case, self._ptrs(Q), self._ptrs(out), N.ptr(dtt.data_ptr()),
                                      float(time), self._stream()), "wm_advance")
         return out
 
@@ -298,7 +299,7 @@ class Solver:
         dt_next = torch.empty((), dtype=torch.float64, device=self.device)
         out = tuple(torch.empty_like(q) for q in Q)
         N.check(self._lib.wm_step_fused(self._case, self._ptrs(Q), self._ptrs(out),
-                                        N.ptr_array([dt.data_ptr()])[0], N.ptr_array([dt_next.data_ptr()])[0],
+                                        N.ptr(dt.data_ptr()), N.ptr(dt_next.data_ptr()),
                                         float(time), self._stream()), "wm_step_fused")
         self._chain = (tuple((weakref.ref(q), q._version) for q in out), dt_next)
         return out, dt
