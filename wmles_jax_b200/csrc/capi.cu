@@ -442,26 +442,28 @@ int extruded_tables(wm_case* c, BlockDev& B, int precision) {
         kt[2 * k + 1] = id[k];
         if (!(kt[2 * k] > 0.0)) return WM_OK;
     }
-    double* d_kt = nullptr;
-    int *flag = nullptr, ok = 1;
+    // two allocations (each costs the driver a call that may take long), kept also when the check fails: a
+    // cudaFree here would wait for the device.  The first: the table, the check's flag, the rounded table
+    const size_t nk = kt.size(), nr = (size_t)B.N[0] * B.N[1] * RT_N;
+    const bool mixed = precision == WM_PREC_MIXED;
+    int ok = 1;
+    kt.resize(nk + 1 + (mixed ? (nk + 1) / 2 : 0));
+    std::memcpy(&kt[nk], &ok, sizeof(ok));
+    double *d_kt = nullptr, *rows = nullptr;
     int r;
-    if ((r = c->mem.upload(&flag, &ok, 1))) return r;      // kept: a cudaFree here would wait for the device
     if ((r = c->mem.upload(&d_kt, kt.data(), kt.size()))) return r;
+    int* flag = reinterpret_cast<int*>(d_kt + nk);
     CK(launch_ext_check(B.met, B.N, B.ng, k0, d_kt, 16 * 2.220446049250313e-16, flag, 0));
     CK(cudaMemcpy(&ok, flag, sizeof(int), cudaMemcpyDeviceToHost));
     if (!ok) return WM_OK;
-    double* rows = nullptr;
-    const size_t nr = (size_t)B.N[0] * B.N[1] * RT_N;
-    if ((r = c->mem.alloc(&rows, nr))) return r;
+    if ((r = c->mem.alloc(&rows, nr + (mixed ? nr / 2 : 0)))) return r;
     CK(launch_ext_rows(B.met, B.N, k0, rows, 0));
     B.rows = rows;
     B.ktab = d_kt;
-    if (precision == WM_PREC_MIXED) {
-        float *rows32 = nullptr, *kt32 = nullptr;
-        if ((r = c->mem.alloc(&rows32, nr))) return r;
-        if ((r = c->mem.alloc(&kt32, kt.size()))) return r;
+    if (mixed) {
+        float *rows32 = reinterpret_cast<float*>(rows + nr), *kt32 = reinterpret_cast<float*>(d_kt + nk + 1);
         CK(launch_to_f32(rows, rows32, (long long)nr, 0));
-        CK(launch_to_f32(d_kt, kt32, (long long)kt.size(), 0));
+        CK(launch_to_f32(d_kt, kt32, (long long)nk, 0));
         B.rows32 = rows32;
         B.ktab32 = kt32;
     }
