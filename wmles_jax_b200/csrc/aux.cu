@@ -155,11 +155,11 @@ __global__ void __launch_bounds__(DT_NT, EXT || sizeof(M) == 4 ? 4 : 3) dt_kerne
             for (int v = 0; v < 5; ++v) qv[v] = q[v * N + idx];
             // every metric this cell needs, read-only and issued before any store to q.  Blocks extruded
             // along k: from the (i, j) row (one line for all of a row's cells) and the factor per k, values
-            // that stay in L1, instead of 18 loads per cell.  S: mean areas of the three directions (float
-            // form: lower and upper, summed below in the general order)
+            // that stay in L1, instead of 18 loads per cell.  S: lower plus upper area of the three directions, added as they
+            // arrive (kept apart, they spilled in FP64: channel 88 us a pass instead of 79)
             const bool ext = EXT || B.rows != nullptr;
             constexpr bool RATE = sizeof(M) == 8;        // FP64: the extruded blocks' own rate
-            M Sl[9], Sh[9], mi = M(0), mj = M(0), rk = M(1);
+            M S[9], mi = M(0), mj = M(0), rk = M(1);
             if (ext) {
                 const M* row = rows_of<M>(B) + ((long long)i * B.N[1] + j) * RT_N;
                 rk = __ldg(ktab_of<M>(B) + 2 * k);
@@ -170,23 +170,18 @@ __global__ void __launch_bounds__(DT_NT, EXT || sizeof(M) == 4 ? 4 : 3) dt_kerne
                 }
 #pragma unroll
                 for (int x = 0; x < 2; ++x) {
-                    Sl[x] = __ldg(row + RT_SI + x) * rk;
-                    Sh[x] = __ldg(row + RT_HI + x) * rk;
-                    Sl[3 + x] = __ldg(row + RT_SJ + x) * rk;
-                    Sh[3 + x] = __ldg(row + RT_N + RT_SJ + x) * rk;
-                    Sl[6 + x] = Sh[6 + x] = M(0);
-                    Sl[2 + 3 * x] = Sh[2 + 3 * x] = M(0);
+                    S[x] = __ldg(row + RT_SI + x) * rk + __ldg(row + RT_HI + x) * rk;
+                    S[3 + x] = __ldg(row + RT_SJ + x) * rk + __ldg(row + RT_N + RT_SJ + x) * rk;
+                    S[6 + x] = S[2 + 3 * x] = M(0);
                 }
-                Sl[8] = Sh[8] = sk;
+                S[8] = sk + sk;
             } else {
                 const int off[3] = {plane, Nk, 1};
 #pragma unroll
                 for (int d = 0; d < 3; ++d)
 #pragma unroll
-                    for (int x = 0; x < 3; ++x) {
-                        Sl[3 * d + x] = __ldg(met + (3 * d + x) * N + idx);
-                        Sh[3 * d + x] = __ldg(met + (3 * d + x) * N + idx + off[d]);
-                    }
+                    for (int x = 0; x < 3; ++x)
+                        S[3 * d + x] = __ldg(met + (3 * d + x) * N + idx) + __ldg(met + (3 * d + x) * N + idx + off[d]);
             }
             // V, or 1/V for the extruded blocks' FP64 rate
             const M vol = __ldg(met + ((RATE && ext ? WM_MET_IVOL : WM_MET_VOL) * N + idx));
@@ -215,13 +210,13 @@ __global__ void __launch_bounds__(DT_NT, EXT || sizeof(M) == 4 ? 4 : 3) dt_kerne
                 // FP64, extruded: the same rate with one root and two divisions after 1 / rho (instead of
                 // five and three): the mean areas' lengths come with the row, the speed of sound from
                 // sqrt(T / T_ref), and cfl V / (lam + 4 nu S2 / V) is cfl / (iv (lam + 4 nu S2 iv)).
-                // Channel 256 x 128 x 128, with the rows' areas and the descriptors in shared memory: 134 ->
-                // 91 us a pass (float form 110 -> 92, its rate unchanged)
+                // Channel 256 x 128 x 128, with the rows' areas, the descriptors in shared memory and no
+                // spills: 134 -> 79 us a pass (float form 110 -> 81, its rate unchanged)
                 const double iv = vol, T = p * ir * P.inv_Rg, x = T * P.inv_Tref, rx = sqrt(x);
                 const double nu = P.nu_fac * (P.mu_ref * (x * rx) * P.TrefS / (T + P.S_suth)) * ir;
-                const double sk = fabs(Sl[8]);
-                const double lam = (fabs(u * (0.5 * (Sl[0] + Sh[0])) + v * (0.5 * (Sl[1] + Sh[1]))) +
-                                    fabs(u * (0.5 * (Sl[3] + Sh[3])) + v * (0.5 * (Sl[4] + Sh[4])))) +
+                const double sk = fabs(0.5 * S[8]);
+                const double lam = (fabs(u * (0.5 * S[0]) + v * (0.5 * S[1])) +
+                                    fabs(u * (0.5 * S[3]) + v * (0.5 * S[4]))) +
                                    fabs(w) * sk + P.c_ref * rx * ((mi + mj) + sk);
                 const double s2 = (mi * mi + mj * mj) + sk * sk;
                 run = nanmin(run, P.cfl / (iv * (lam + 4.0 * nu * s2 * iv)));
@@ -240,9 +235,9 @@ __global__ void __launch_bounds__(DT_NT, EXT || sizeof(M) == 4 ? 4 : 3) dt_kerne
                 CF lam = CF(0), lamv = CF(0);
 #pragma unroll
                 for (int d = 0; d < 3; ++d) {
-                    const CF sx = CF(0.5) * (Sl[3 * d] + Sh[3 * d]);
-                    const CF sy = CF(0.5) * (Sl[3 * d + 1] + Sh[3 * d + 1]);
-                    const CF sz = CF(0.5) * (Sl[3 * d + 2] + Sh[3 * d + 2]);
+                    const CF sx = CF(0.5) * S[3 * d];
+                    const CF sy = CF(0.5) * S[3 * d + 1];
+                    const CF sz = CF(0.5) * S[3 * d + 2];
                     const CF Sm = sqrt((sx * sx + sy * sy) + sz * sz);
                     lam = lam + fabs((uc * sx + vc * sy) + wc * sz) + cs * Sm;
                     lamv = lamv + nu * (Sm * Sm) * ivol;
