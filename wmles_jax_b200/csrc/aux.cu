@@ -90,8 +90,10 @@ struct DtPhys {
 // one atomicMin on the case's key.  The last CTA to finish turns the keys into time steps
 // and resets them.  A minimum is exact in any order, so the result does not depend on the
 // grid, the chunking or the batch.  M: the metric copy read (double; float for the mixed
-// form).  EXT: every block of the view is extruded along k (the same arithmetic for such a block as
-// in the other instance, without the registers of the general form).
+// form).  EXT: the launch takes the view's blocks that are extruded along k, the other instance the
+// general ones; a view with both kinds has two launches.  A block's rate is so computed by the same
+// code whatever else is in the view, and the general instance does not carry the rows' branch
+// (192 x 112 x 96 FP64: 62 us a call of max_dt with it, 54 without).
 template <typename M, bool EXT>
 __global__ void __launch_bounds__(DT_NT, EXT || sizeof(M) == 4 ? 4 : 3) dt_kernel(const __grid_constant__ DtArgs D) {
     chain_wait();
@@ -157,10 +159,9 @@ __global__ void __launch_bounds__(DT_NT, EXT || sizeof(M) == 4 ? 4 : 3) dt_kerne
             // along k: from the (i, j) row (one line for all of a row's cells) and the factor per k, values
             // that stay in L1, instead of 18 loads per cell.  S: lower plus upper area of the three directions, added as they
             // arrive (kept apart, they spilled in FP64: channel 88 us a pass instead of 79)
-            const bool ext = EXT || B.rows != nullptr;
-            constexpr bool RATE = sizeof(M) == 8;        // FP64: the extruded blocks' own rate
+            constexpr bool RATE = EXT && sizeof(M) == 8;     // FP64: the extruded blocks' own rate
             M S[9], mi = M(0), mj = M(0), rk = M(1);
-            if (ext) {
+            if constexpr (EXT) {
                 const M* row = rows_of<M>(B) + ((long long)i * B.N[1] + j) * RT_N;
                 rk = __ldg(ktab_of<M>(B) + 2 * k);
                 const M sk = __ldg(row + RT_SK);
@@ -184,7 +185,7 @@ __global__ void __launch_bounds__(DT_NT, EXT || sizeof(M) == 4 ? 4 : 3) dt_kerne
                         S[3 * d + x] = __ldg(met + (3 * d + x) * N + idx) + __ldg(met + (3 * d + x) * N + idx + off[d]);
             }
             // V, or 1/V for the extruded blocks' FP64 rate
-            const M vol = __ldg(met + ((RATE && ext ? WM_MET_IVOL : WM_MET_VOL) * N + idx));
+            const M vol = __ldg(met + ((RATE ? WM_MET_IVOL : WM_MET_VOL) * N + idx));
             if (cmf) {
                 const double delta = D.cmf_delta[B.case_id];
                 const int m = 1 + C.cmf_dir;
@@ -206,7 +207,7 @@ __global__ void __launch_bounds__(DT_NT, EXT || sizeof(M) == 4 ? 4 : 3) dt_kerne
                 if (!(p > 0.0)) bad |= WM_ST_PRESSURE;
                 if (bad) atomicOr(C.status, bad);
             }
-            if (RATE && ext && D.want_dt) {
+            if (RATE && D.want_dt) {
                 // FP64, extruded: the same rate with one root and two divisions after 1 / rho (instead of
                 // five and three): the mean areas' lengths come with the row, the speed of sound from
                 // sqrt(T / T_ref), and cfl V / (lam + 4 nu S2 / V) is cfl / (iv (lam + 4 nu S2 iv)).
@@ -279,6 +280,7 @@ __global__ void __launch_bounds__(DT_NT, EXT || sizeof(M) == 4 ? 4 : 3) dt_kerne
     }
     if (!D.want_dt) return;
     if (cur >= 0) flush();
+    if (!D.finish) return;         // the view's general blocks; the launch after this one finishes
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();

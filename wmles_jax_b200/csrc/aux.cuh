@@ -29,7 +29,8 @@ struct DtArgs {
     const CaseDev* cases;
     int nblocks;
     int ncta;                              // chunks of DT_NT interior cells, numbered block by block
-    int cta_start[WM_MAX_BLOCKS + 1];      // chunks of block b: [cta_start[b], cta_start[b+1])
+    int cta_start[WM_MAX_BLOCKS + 1];      // chunks of block b: [cta_start[b], cta_start[b+1]) (none for
+                                           // the blocks of the other kind)
     int ncases;
     int case_block_start[MAX_CASES + 1];   // blocks of case c: [start[c], start[c+1])
     double* q[WM_MAX_BLOCKS];      // state (modified in place when the constraint is applied)
@@ -42,7 +43,8 @@ struct DtArgs {
     const double* cmf_delta;       // per case: constant-mass-flux shift from stage 3 (null: none)
     int want_dt;                   // 0: constraint only
     int met32;                     // read the float metric copy (mixed form)
-    int ext;                       // every block is extruded along k
+    int ext;                       // the launch takes the blocks extruded along k, else the general ones
+    int finish;                    // the pass's last launch: turns the minima into time steps
     unsigned long long* dt_key;    // per case: running minimum as an order-preserving key
                                    // (DT_KEY_EMPTY between calls: reset by the last CTA)
     unsigned int* counter;         // last-CTA-done counter (reset by the last CTA)

@@ -201,7 +201,8 @@ struct View {
     double *cmf_part = nullptr, *cmf_delta = nullptr;
     unsigned long long* dt_key = nullptr;   // CFL pass: per-case minimum keys
     unsigned* counters = nullptr;        // [0]: CFL reduction, [1]: constant-mass-flux reduction
-    std::vector<int> cta_start;          // CFL pass: first CTA of each view block (+ total)
+    std::vector<int> cta_start[2];       // CFL pass of the general and of the extruded blocks: first chunk of
+                                         // each view block (+ total)
     std::vector<int> gcta_start;         // same for the blocks' ghost cells (output ghost fill)
     int max_wall_faces = 0;
     std::vector<int> sp_rows;            // (view block, row) pairs of the sponge rows of every case
@@ -534,10 +535,12 @@ int build_view(View* v, wm_case* const* cases, int n) {
         build_waves(v->hb, &w, stage_slots(v->opts));
     }
     cmf_slots(v);
-    v->cta_start.assign(1, 0);                  // one interior cell per thread of the CFL pass
+    for (std::vector<int>& start : v->cta_start) start.assign(1, 0);   // one interior cell per thread of the CFL pass
     v->gcta_start.assign(1, 0);                 // one ghost cell per thread
     for (const BlockDev& B : v->hb) {
-        v->cta_start.push_back(v->cta_start.back() + (int)(((long long)B.n[0] * B.n[1] * B.n[2] + DT_NT - 1) / DT_NT));
+        const int chunks = (int)(((long long)B.n[0] * B.n[1] * B.n[2] + DT_NT - 1) / DT_NT);
+        for (int x = 0; x < 2; ++x)
+            v->cta_start[x].push_back(v->cta_start[x].back() + (x == (B.rows ? 1 : 0) ? chunks : 0));
         v->gcta_start.push_back(v->gcta_start.back() + (int)((ghost_cells(B) + DT_NT - 1) / DT_NT));
     }
     int r;
@@ -656,9 +659,6 @@ int run_dt(View* v, Prof* pf, double* const* q, bool apply_cmf, bool want_dt, do
            const double* const* q_src, cudaStream_t s) {
     DtArgs D{};
     D.blocks = v->d_blocks; D.cases = v->d_cases; D.nblocks = v->nblocks;
-    D.ncta = v->cta_start.back();
-    for (int b = 0; b <= v->nblocks; ++b) D.cta_start[b] = v->cta_start[b];
-    D.ngcta = q_src ? v->gcta_start.back() : 0;
     for (int b = 0; b <= v->nblocks; ++b) D.gcta_start[b] = v->gcta_start[b];
     for (int b = 0; b < v->nblocks; ++b) D.q_src[b] = q_src ? q_src[b] : nullptr;
     D.ncases = v->ncases;
@@ -667,11 +667,19 @@ int run_dt(View* v, Prof* pf, double* const* q, bool apply_cmf, bool want_dt, do
     D.cmf_delta = apply_cmf ? v->cmf_delta : nullptr;
     D.want_dt = want_dt ? 1 : 0;
     D.met32 = v->opts.precision == WM_PREC_MIXED ? 1 : 0;
-    D.ext = v->work[0].blocks.empty() ? 1 : 0;
     D.dt_key = v->dt_key; D.counter = v->counters;
     for (int ci = 0; ci < v->ncases; ++ci) D.dt_out[ci] = dt_out ? dt_out[ci] : nullptr;
-    LaunchScope ls(pf, WM_KIND_DT, s);
-    CK(launch_dt(D, s));
+    // one launch per kind of block in the view; the ghost cells ride on the last
+    for (int x = 0; x < 2; ++x) {
+        if (v->work[x].blocks.empty()) continue;
+        D.ext = x;
+        D.finish = x == 1 || v->work[1].blocks.empty() ? 1 : 0;
+        D.ncta = v->cta_start[x].back();
+        for (int b = 0; b <= v->nblocks; ++b) D.cta_start[b] = v->cta_start[x][b];
+        D.ngcta = q_src && D.finish ? v->gcta_start.back() : 0;
+        LaunchScope ls(pf, WM_KIND_DT, s);
+        CK(launch_dt(D, s));
+    }
     return WM_OK;
 }
 
@@ -1118,11 +1126,11 @@ int wm_batch_info(wm_batch* b, int* nblocks, int* ntiles, long long* launches_pe
     const View& v = b->view;
     int inflow = 0;
     for (wm_case* c : v.members) inflow += c->has_inflow ? 1 : 0;
-    const long long per_stage = IN_LAUNCHES * inflow + ((v.total_rhs || !v.hw.empty() || v.any_sponge) ? 1 : 0) +
-                                (v.work[0].tiles.empty() ? 0 : 1) + (v.work[1].tiles.empty() ? 0 : 1);
+    const int kinds = (v.work[0].tiles.empty() ? 0 : 1) + (v.work[1].tiles.empty() ? 0 : 1);
+    const long long per_stage = IN_LAUNCHES * inflow + ((v.total_rhs || !v.hw.empty() || v.any_sponge) ? 1 : 0) + kinds;
     if (nblocks) *nblocks = v.nblocks;
     if (ntiles) *ntiles = (int)(v.work[0].tiles.size() + v.work[1].tiles.size());
-    if (launches_per_step) *launches_per_step = 3 * per_stage + 1;
+    if (launches_per_step) *launches_per_step = 3 * per_stage + kinds;
     return WM_OK;
 }
 
