@@ -137,7 +137,7 @@ typedef struct {
     wm_sponge sponge;
     int tile;                 /* stage-kernel tile shape id (0 = 8x32, 1 = 16x16, 2 = 4x32,
                                  3 = 16x32, mixed form only); -1 = automatic: a shape per
-                                 block from its extents */
+                                 block from its extents and its share of the GPU */
     int chunk;                /* planes per CTA along i, 0 = automatic */
 } wm_case_desc;
 

@@ -2,7 +2,7 @@
 
 The stage kernel marches a TJ x TK column of cells along i (tile ids: 0 = 8x32, 1 = 16x16,
 2 = 4x32, 3 = 16x32, the last built for the mixed form only; -1 = a shape per block from its
-extents, the default).  Which shape is fastest depends
+extents and its share of the GPU, the default).  Which shape is fastest depends
 on the grid extents (partial tiles at the j/k edges, waves of CTAs over the SMs), on the
 precision (registers and shared memory decide CTAs per SM) and on the scheme.  ``tune``
 measures it: for each candidate tile it builds the cases with that tile, advances them
@@ -10,10 +10,10 @@ together (one batched step, as the server runs them) and times the steps with CU
 the fastest tile is stored in a JSON cache keyed by GPU name, precision, scheme, SGS model
 and the block extents of the workload, so each workload is tuned once per machine.
 
-The tile shape does not change the physics; it does change the summation order of the
-stage-3 mass-flux partials, so results with different tiles agree to round-off, not bitwise.
-A server therefore fixes one tile for all its cases (``Server(tile="auto")`` tunes it over
-its grid mix before serving).
+The tile shape does not change the physics; ids 0-2 and 3 / -1 of the mixed form are different
+kernel instances, whose results agree to round-off, not bitwise.  A server therefore
+fixes one tile for all its cases (``Server(tile="auto")`` tunes it over its grid mix before
+serving).
 """
 import copy
 import json

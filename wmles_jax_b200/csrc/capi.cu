@@ -6,10 +6,9 @@
 // reduction scratch of a set of cases.  Every wm_case carries a View of itself for the
 // single-case entry points; a wm_batch is a View over several resident cases, so one
 // launch per kernel and stage advances all of them.  The stage work list is cut for the
-// whole view (longer chunks along i when many cases share the GPU).  Per-case reductions
-// (CFL minimum; constant-mass-flux sum over fixed per-column, per-plane partials)
-// run in a fixed order, so a case's result depends neither on the chunk length nor on what
-// else is in the batch.
+// whole view (tile shapes and chunks along i by how many cases share the GPU).  Per-case
+// reductions are exact in any order (CFL minimum; constant-mass-flux sum in bins), so a case's
+// result depends neither on the tiles nor on what else is in the batch.
 #include <algorithm>
 #include <cmath>
 #include <cstdarg>
@@ -190,15 +189,13 @@ struct View {
         int ctas() const { return cta_first.empty() ? (int)tiles.size() : (int)cta_first.size() - 1; }
     } work[2];
     std::vector<int> case_block_start;
-    std::vector<int> cmf_slot_start, case_slot_start;   // constant-mass-flux partial slots
     std::vector<GhostSeg> seg_rhs, seg_all;
     int total_rhs = 0, total_all = 0;
     BlockDev* d_blocks = nullptr;
     CaseDev* d_cases = nullptr;
     WallDev* d_walls = nullptr;
-    int* d_case_slot_start = nullptr;
     GhostSeg *d_seg_rhs = nullptr, *d_seg_all = nullptr;
-    double *cmf_part = nullptr, *cmf_delta = nullptr;
+    double *cmf_sum = nullptr, *cmf_delta = nullptr;   // constant mass flux: per case three sums, the shift
     unsigned long long* dt_key = nullptr;   // CFL pass: per-case minimum keys
     unsigned* counters = nullptr;        // [0]: CFL reduction, [1]: constant-mass-flux reduction
     std::vector<int> cta_start[2];       // CFL pass of the general and of the extruded blocks: first chunk of
@@ -316,9 +313,7 @@ long long columns(const BlockDev& B) {
 
 // the tile of a block's column at (j0, k0) over planes [i0, i1)
 Tile make_tile(const BlockDev& B, int b, int j0, int k0, int i0, int i1) {
-    const int colk = (B.n[2] + B.tk - 1) / B.tk;
-    return Tile{b, j0, k0, i0, i1, std::min(B.tj, B.ng + B.n[1] - j0), std::min(B.tk, B.ng + B.n[2] - k0),
-                ((j0 - B.ng) / B.tj) * colk + (k0 - B.ng) / B.tk};
+    return Tile{b, j0, k0, i0, i1, std::min(B.tj, B.ng + B.n[1] - j0), std::min(B.tk, B.ng + B.n[2] - k0)};
 }
 
 // planes per stage-kernel CTA: wave quantisation against the chunk prologue cost
@@ -392,16 +387,39 @@ void build_waves(const std::vector<BlockDev>& hb, View::Work* v, int slots) {
     }
 }
 
-// constant-mass-flux partial slots of a view: one per (column, interior plane) of each block,
-// independent of how the columns are cut into CTAs
-void cmf_slots(View* v) {
-    v->cmf_slot_start.assign(1, 0);
-    for (int b = 0; b < v->nblocks; ++b) {
-        const BlockDev& B = v->hb[b];
-        v->cmf_slot_start.push_back(v->cmf_slot_start.back() + (int)columns(B) * B.n[0]);
+// Rounding constants of a case's sum of rho u V (constant mass flux), one per bin: 3 x 2^51 u, so that
+// x + c - c is x to a multiple of u.  The bins take a value apart, each what the one above left over:
+// |x| < 2^e and fewer than 2^n cells make every sum of the first bin's parts a multiple of u = 2^(e+n-52)
+// below 2^53 u, which FP64 adds without rounding, so in any order to the same bits; the parts left over are below u / 2,
+// and the next bin has u 2^(n-53).  What the third leaves is under 2^(e + 3 n - 158) a cell, for 2^22 cells and a
+// total of 2^-30 x 2^e a cell some 2^-62 of the total.  2^e is 2^30 times the mean cell's volume times the
+// target or, where that is larger (a target of zero), the speed of sound; values beyond it are still added,
+// but rounded, as any sum is.
+void cmf_bins(CaseDev& C, double cells) {
+    int n, e;
+    std::frexp(std::max(cells, 8.0), &n);
+    const double c = std::isfinite(C.c_ref) ? C.c_ref : 0.0;
+    std::frexp(std::max(std::fabs(C.cmf_target), c) * (C.cmf_volume / cells), &e);
+    for (int m = 0, u = e + 30 + n - 52; m < 3; ++m, u += n - 53) C.cmf_bin[m] = std::ldexp(3.0, u + 51);
+}
+
+// Tile shapes of a view: the blocks of like extents on their share of the GPU, among those of a launch.  A case's results do
+// not depend on them, so that it has one shape alone and another among many: 64 channels of 16^3
+// in a batch, float form, took 736 us a step with the shapes of the cases alone and 210 with the batch's.
+void view_tiles(std::vector<BlockDev>& hb, const std::vector<int>& blocks, const StageOpts& opts, int slots) {
+    double cells = 0.0;
+    auto size = [](const BlockDev& B) { return (double)B.n[0] * B.n[1] * B.n[2]; };
+    for (int b : blocks) cells += size(hb[b]);
+    for (int b : blocks) hb[b].tj = 0;
+    for (int b : blocks) {
+        if (hb[b].tj) continue;
+        auto same = [&](int o) { return std::equal(hb[b].n, hb[b].n + 3, hb[o].n); };
+        const int count = (int)std::count_if(blocks.begin(), blocks.end(), same);
+        int tj, tk;
+        tile_shape(opts, hb[b].n, count, (int)(slots * (count * size(hb[b]) / cells) + 0.5), &tj, &tk);
+        for (int o : blocks)
+            if (same(o)) { hb[o].tj = tj; hb[o].tk = tk; }
     }
-    v->case_slot_start.clear();
-    for (int c = 0; c <= v->ncases; ++c) v->case_slot_start.push_back(v->cmf_slot_start[v->case_block_start[c]]);
 }
 
 // chunked split: every column cut into chunks of ic planes, one chunk per CTA
@@ -529,12 +547,12 @@ int build_view(View* v, wm_case* const* cases, int n) {
     for (int b = 0; b < v->nblocks; ++b) v->work[v->hb[b].rows ? 1 : 0].blocks.push_back(b);
     for (View::Work& w : v->work) {
         if (w.blocks.empty()) continue;
+        view_tiles(v->hb, w.blocks, v->opts, stage_slots(v->opts));
         const int ic = choose_chunk(v->hb, w.blocks, v->opts, req);
         build_tiles(v->hb, &w, ic);
         if (req != 0) continue;
         build_waves(v->hb, &w, stage_slots(v->opts));
     }
-    cmf_slots(v);
     for (std::vector<int>& start : v->cta_start) start.assign(1, 0);   // one interior cell per thread of the CFL pass
     v->gcta_start.assign(1, 0);                 // one ghost cell per thread
     for (const BlockDev& B : v->hb) {
@@ -553,14 +571,13 @@ int build_view(View* v, wm_case* const* cases, int n) {
         if (!w.cta_first.empty())
             if ((r = m.upload(&w.d_cta_first, w.cta_first.data(), w.cta_first.size()))) return r;
     }
-    if ((r = m.upload(&v->d_case_slot_start, v->case_slot_start.data(), v->case_slot_start.size()))) return r;
     if ((r = m.upload(&v->d_seg_rhs, v->seg_rhs.data(), v->seg_rhs.size()))) return r;
     if ((r = m.upload(&v->d_seg_all, v->seg_all.data(), v->seg_all.size()))) return r;
     if (!v->sp_rows.empty())
         if ((r = m.upload(&v->d_sp_rows, v->sp_rows.data(), v->sp_rows.size()))) return r;
-    if ((r = m.alloc(&v->cmf_part, (size_t)v->cmf_slot_start.back()))) return r;
-    if ((r = m.alloc(&v->cmf_delta, (size_t)n))) return r;
-    CK(cudaMemset(v->cmf_delta, 0, sizeof(double) * n));
+    if ((r = m.alloc(&v->cmf_sum, 4 * (size_t)n))) return r;
+    v->cmf_delta = v->cmf_sum + 3 * (size_t)n;
+    CK(cudaMemset(v->cmf_sum, 0, sizeof(double) * 4 * n));
     {
         const std::vector<unsigned long long> empty((size_t)n, DT_KEY_EMPTY);
         if ((r = m.upload(&v->dt_key, empty.data(), empty.size()))) return r;
@@ -628,8 +645,7 @@ int run_stage(View* v, Prof* pf, int stage, double* const* q_in, const double* c
     A.cmf_ctas = v->work[0].ctas() + v->work[1].ctas();
     A.stage = stage;
     A.ncases = v->ncases;
-    A.case_slot_start = v->d_case_slot_start;
-    A.cmf_part = (stage == 3 && v->any_cmf) ? v->cmf_part : nullptr;
+    A.cmf_sum = (stage == 3 && v->any_cmf) ? v->cmf_sum : nullptr;
     A.cmf_counter = v->counters + 1;
     A.cmf_delta = v->cmf_delta;
     for (int ci = 0; ci < v->ncases; ++ci) A.dt[ci] = dt ? dt[ci] : nullptr;
@@ -638,13 +654,12 @@ int run_stage(View* v, Prof* pf, int stage, double* const* q_in, const double* c
         A.p[b].q0 = q0 ? q0[b] : q_in[b];
         A.p[b].q_out = q_out[b];
         A.p[b].spmean = spm[b];
-        A.cmf_slot_start[b] = v->cmf_slot_start[b];
     }
     for (int x = 0; x < 2; ++x) {
         const View::Work& w = v->work[x];
         if (w.tiles.empty()) continue;
         A.ext = x;
-        A.tiles = w.d_tiles; A.ntiles = (int)w.tiles.size();
+        A.tiles = w.d_tiles;
         A.cta_first = w.d_cta_first;
         A.nctas = w.ctas();
         LaunchScope ls(pf, WM_KIND_STAGE, s);
@@ -779,14 +794,14 @@ int wm_case_create(const wm_case_desc* d, wm_case** out) {
         C.sp_invL = 1.0 / d->sponge.L;
     }
     // automatic tile (-1): one kernel variant per precision (so cases created with the default
-    // can share a batch), the tile shape chosen per block from the case's extents alone
+    // can share a batch), the tile shape chosen per block and view (view_tiles)
     c->opts = StageOpts{d->precision, d->scheme, d->kep_order, d->limiter, d->sgs, d->tile < 0 ? -1 : d->tile};
 
     // ---- blocks, metrics, work buffers
     c->hb.resize(d->nblocks);
-    const int slots = stage_slots(c->opts);
     double cells = 0.0;
     for (int b = 0; b < d->nblocks; ++b) cells += (double)d->blocks[b].n[0] * d->blocks[b].n[1] * d->blocks[b].n[2];
+    if (C.cmf_dir >= 0) cmf_bins(C, cells);
     for (int b = 0; b < d->nblocks; ++b) {
         const wm_block& src = d->blocks[b];
         BlockDev& B = c->hb[b];
@@ -798,8 +813,6 @@ int wm_case_create(const wm_case_desc* d, wm_case** out) {
         for (int f = 0; f < 6; ++f) B.wall[f] = -1;
         B.div_nj.set(B.n[1]);
         B.div_nk.set(B.n[2]);
-        // each block on its share of the GPU
-        tile_shape(c->opts, B.n, (int)(slots * ((double)B.n[0] * B.n[1] * B.n[2] / cells) + 0.5), &B.tj, &B.tk);
         if (B.ncell * WM_NMET >= (1LL << 31))
             return bail(fail(WM_E_UNSUPPORTED, "block %d: %lld cells exceed the 32-bit metric index range "
                              "(split the block)", b, B.ncell));

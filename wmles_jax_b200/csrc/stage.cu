@@ -19,8 +19,8 @@
 // Float form: three phases, conversion of plane i+1; gradient records; faces and the RK
 // epilogue of plane i-1.
 // Each face flux is evaluated once; each conservative value is read from HBM about once
-// per stage (halo re-reads hit L2).  Stage 3 also emits per-(column, plane) partial sums of
-// rho u V for the constant-mass-flux constraint.
+// per stage (halo re-reads hit L2).  Stage 3 also sums rho u V for the constant-mass-flux
+// constraint.
 //
 // Reference: Solver._block_rhs (wmles/solver.py:76-95), green_gauss / viscous_flux /
 // ducros (wmles/viscous.py), schemes (wmles/schemes.py), SGS (wmles/sgs.py), SSP-RK3
@@ -49,8 +49,6 @@ namespace wm {
 // and j faces.  Their metrics come from a row of 16 values per (i, j), staged for the tile's
 // rows one plane ahead, and a pair of values per k; only 1/V and the filter width are read
 // per cell.
-constexpr int STAGE_MAX_WARPS = 32;          // two reduction sums per warp in the scratch
-
 template <typename R, int SCHEME, int CAP, bool EXT>
 struct StageLayout {
     static constexpr int NTH = sizeof(R) == 8 ? 512 : (CAP == 512 ? 640 : 256);     // threads
@@ -89,7 +87,9 @@ struct StageLayout {
     static constexpr size_t hp_off = fr_off + (FUSE ? sizeof(R) * 5 * CAP : 0);        // R [HP_N][CAP]
     static constexpr size_t hg_off = hp_off + (FUSE ? sizeof(R) * HP_N * CAP : 0);     // R [NGS][CAP]
     static constexpr size_t red_off = (hg_off + (FUSE && !PING ? sizeof(R) * NGS * CAP : 0) + 15) / 16 * 16;
-    static constexpr size_t rt_off = red_off + sizeof(double) * 2 * STAGE_MAX_WARPS;   // R [2][RN][RT_N]
+    // mass-flux sums of the warps (three bins each), the bins' rounding constants
+    static constexpr size_t cs_off = red_off + (sizeof(double) * 3 * (NTH / 32 + 1) + 15) / 16 * 16;   // float form: double [3][CAP]
+    static constexpr size_t rt_off = cs_off + (FUSE ? 0 : sizeof(double) * 3 * CAP);                   // R [2][RN][RT_N]
     static constexpr size_t kt_off = rt_off + sizeof(R) * 2 * RN * RT_N;               // R [KN][2]
     // index tables of the segment
     static constexpr size_t ft_off = kt_off + sizeof(R) * 2 * KN;                      // int [FN]
@@ -97,7 +97,6 @@ struct StageLayout {
     static constexpr size_t ct_off = pt_off + 4 * PN;                                  // int [CAP]
     static constexpr size_t ph_off = (ct_off + 4 * CAP + 7) / 8 * 8;                   // Phys<R>
     static constexpr size_t bytes = ph_off + (sizeof(Phys<R>) + 7) / 8 * 8;
-    static_assert(NTH / 32 <= STAGE_MAX_WARPS, "the reduction scratch holds two sums per warp");
     static constexpr int GW = (GN + 31) / 32 * 32;     // threads of the warps with a record, at most
     static_assert(!FUSE || 2 * (NTH - GW) >= CAP, "at most two epilogue columns per thread");
     static_assert(rt_off % 16 == 0, "rows arrive in 16-byte pieces");
@@ -603,14 +602,20 @@ __device__ __forceinline__ void stage_segment(const StageArgs& A, const StageOpt
     };
 
     const double dt = A.stage ? *A.dt[B.case_id] : 0.0;
-    // constant mass flux (stage 3): one partial of rho u_dir V per (tile column, plane) -
-    // the warps' sums of the plane added in warp order in shared memory - so the case's sum
-    // does not depend on how the columns are cut into chunks along i
-    const bool cmf_on = A.stage == 3 && A.cmf_part != nullptr && C.cmf_dir >= 0;
+    // constant mass flux (stage 3): sum of rho u_dir V over the case, exact in three bins of fixed
+    // exponent (cmf_bins, capi.cu), so that its bits depend neither on the tiles' shape nor on the order
+    // in which threads, CTAs and launches add.  The sums wait in shared memory (in registers they cost some
+    // 50 B of spills): a column's in the float form, a warp's in FP64, which has no room for the columns'
+    // (float form with a warp's: 30 shuffles for every warp and plane, channel 256 x 128 x 128 1188 us a step
+    // against 1158).
+    const bool cmf_on = A.stage == 3 && A.cmf_sum != nullptr && C.cmf_dir >= 0;
     const int cmf_dir = C.cmf_dir;
-    double cmf_acc = 0.0;
-    double* cmf_col = nullptr;
-    if (cmf_on) cmf_col = A.cmf_part + A.cmf_slot_start[t.blk] + (long long)t.col * B.n[0];
+    double* cmf_bin = red + 3 * NW;
+    if (cmf_on && tid < 3 * NW + 3) red[tid] = tid < 3 * NW ? 0.0 : C.cmf_bin[tid - 3 * NW];
+    double* cmf_col = reinterpret_cast<double*>(smem_raw + LY::cs_off) + threadIdx.x;
+    if (!FUSE && cmf_on && tid < CAP)
+#pragma unroll
+        for (int m = 0; m < 3; ++m) cmf_col[m * CAP] = 0.0;
 
     // ---- RK epilogue of one cell: its operands, loaded ahead of use (from issue to use some 2000
     // cycles under load), then r = -(div F)/V (+ source) from the flux divergence dv (times -1,
@@ -630,7 +635,8 @@ __device__ __forceinline__ void stage_segment(const StageArgs& A, const StageOpt
         }
         if (cmf_on) e.vol = __ldg(B.met + WM_MET_VOL * nc + idx);
     };
-    auto output = [&](int io, int c, const Epi& e, const R dv[5]) {
+    // returns rho u_dir V of stage 3 with constant mass flux, else 0
+    auto output = [&](int io, int c, const Epi& e, const R dv[5]) -> double {
         const int jk = ct[c], idx = io * planei + jk;
         R r[5];
 #pragma unroll
@@ -666,22 +672,41 @@ __device__ __forceinline__ void stage_segment(const StageArgs& A, const StageOpt
                 qn[v] = (1.0 / 3.0) * e.q0[v] + (2.0 / 3.0) * (e.q[v] + dt * rq[v]);
                 out[v * nc] = qn[v];
             }
-            if (cmf_on) cmf_acc += (cmf_dir == 0 ? qn[1] : cmf_dir == 1 ? qn[2] : qn[3]) * e.vol;
+            // rounded by itself: contracted with a bin's constant, it would depend on the instance
+            if (cmf_on) return __dmul_rn(cmf_dir == 0 ? qn[1] : cmf_dir == 1 ? qn[2] : qn[3], e.vol);
+        }
+        return 0.0;
+    };
+    // a value's part in bin m; x: what it leaves for the next
+    auto cmf_part = [&](int m, double& x) {
+        const double c = cmf_bin[m], h = __dsub_rn(__dadd_rn(x, c), c);
+        x = __dsub_rn(x, h);
+        return h;
+    };
+    auto cmf_warp_sum = [&](int m, double h) {
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) h = __dadd_rn(h, __shfl_down_sync(0xffffffffu, h, off));
+        if ((tid & 31) == 0) red[3 * (tid >> 5) + m] = __dadd_rn(red[3 * (tid >> 5) + m], h);
+    };
+    // FP64: a warp's cells of a plane (up to two a lane)
+    auto cmf_add = [&](double x0, double x1) {
+        constexpr int UNR = SCHEME == WM_SCHEME_HYBRID ? 3 : 1;      // fewest spills
+#pragma unroll UNR
+        for (int m = 0; m < 3; ++m) {
+            const double h = cmf_part(m, x0);
+            cmf_warp_sum(m, __dadd_rn(h, cmf_part(m, x1)));
         }
     };
-    // stage 3's rho u_dir V of a plane: summed per warp; the plane's partial from the sums of warps
-    // [w0, w1), in warp order, after a barrier
-    auto cmf_warp_sum = [&]() {
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) cmf_acc += __shfl_down_sync(0xffffffffu, cmf_acc, off);
-        if ((tid & 31) == 0) red[tid >> 5] = cmf_acc;
-        cmf_acc = 0.0;
-    };
-    auto cmf_store = [&](int io, int w0, int w1) {
-        if (tid == 0) {
-            double sp = 0.0;
-            for (int w = w0; w < w1; ++w) sp += red[w];
-            cmf_col[io - ng] = sp;
+    // the segment's sums into the case's, at its end
+    auto cmf_flush = [&]() {
+        if (!cmf_on) return;
+        if constexpr (!FUSE)
+            for (int m = 0; m < 3; ++m) cmf_warp_sum(m, tid < CAP ? cmf_col[m * CAP] : 0.0);
+        __syncthreads();
+        if (tid < 3) {
+            double sum = 0.0;
+            for (int w = 0; w < NW; ++w) sum = __dadd_rn(sum, red[3 * w + tid]);
+            atomicAdd(A.cmf_sum + 3 * B.case_id + tid, sum);
         }
     };
     // ---- prologue: primitives of planes i0-2, i0-1 (FP64: i0) straight from global memory, the
@@ -770,6 +795,7 @@ __device__ __forceinline__ void stage_segment(const StageArgs& A, const StageOpt
             }
         };
         auto finish = [&](int io) {
+            double x[2] = {0.0, 0.0};
 #pragma unroll
             for (int r = 0; r < 2; ++r) {
                 const int c = ac + r * as;
@@ -777,8 +803,9 @@ __device__ __forceinline__ void stage_segment(const StageArgs& A, const StageOpt
                 R d[5];
 #pragma unroll
                 for (int v = 0; v < 5; ++v) d[v] = fr[v * CAP + c];
-                output(io, c, e[r], d);
+                x[r] = output(io, c, e[r], d);
             }
+            if (cmf_on) cmf_add(x[0], x[1]);
         };
         load_aux(i0 - 2);
 #pragma unroll 1
@@ -803,10 +830,8 @@ __device__ __forceinline__ void stage_segment(const StageArgs& A, const StageOpt
                         for (int v = 0; v < 5; ++v)
                             fr[v * CAP + c] = (pj[v * FN] - pj[v * FN + TK]) * rk - (pk[v * FN + 1] - pk[v * FN]);
                     }
-                if (cmf_on) cmf_warp_sum();
             }
             __syncthreads();
-            if (cmf_on && ip - 2 >= i0) cmf_store(ip - 2, gw >> 5, NW);
             if (!EXT && tid >= CAP && ip < i1) prefetch_next(ip, CAP);
             if (tid >= gw && ip < i1) {
                 stage_rows(ip + 1, gw);
@@ -840,14 +865,8 @@ __device__ __forceinline__ void stage_segment(const StageArgs& A, const StageOpt
             cp_async_wait_all();
             __syncthreads();
         }
-        if (tid >= gw) {
-            finish(i1 - 1);                          // the segment's last plane
-            if (cmf_on) cmf_warp_sum();
-        }
-        if (cmf_on) {
-            __syncthreads();
-            cmf_store(i1 - 1, gw >> 5, NW);
-        }
+        if (tid >= gw) finish(i1 - 1);               // the segment's last plane
+        cmf_flush();
     } else {
         R Flo[5], dv[5];
         Epi e;                                       // operands of the next epilogue
@@ -893,12 +912,16 @@ __device__ __forceinline__ void stage_segment(const StageArgs& A, const StageOpt
             }
             if (column && ip - 1 >= i0) epi_load(ip - 1, tid, e);
             faces(ip);
-            if (column && ip - 1 >= i0) output(ip - 1, tid, e, dv);
-            if (cmf_on) cmf_warp_sum();
+            if (column && ip - 1 >= i0) {
+                double x = output(ip - 1, tid, e, dv);
+                if (cmf_on)
+#pragma unroll
+                    for (int m = 0; m < 3; ++m) cmf_col[m * CAP] = __dadd_rn(cmf_col[m * CAP], cmf_part(m, x));
+            }
             cp_async_wait_all();
             __syncthreads();
-            if (cmf_on && ip - 1 >= i0) cmf_store(ip - 1, 0, NW);
         }
+        cmf_flush();
     }
 }
 
@@ -909,7 +932,6 @@ __global__ void __launch_bounds__(StageLayout<R, SCHEME, CAP, EXT>::NTH, StageLa
     chain_wait();
     constexpr int NTH = LY::NTH;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    double* red = reinterpret_cast<double*>(smem_raw + LY::red_off);
     const int tid = threadIdx.x;
     // this CTA's segments: one tile, or a balanced range of tiles (consecutive column pieces)
     const int first = A.cta_first ? A.cta_first[blockIdx.x] : blockIdx.x;
@@ -920,35 +942,26 @@ __global__ void __launch_bounds__(StageLayout<R, SCHEME, CAP, EXT>::NTH, StageLa
         __syncthreads();                 // shared memory is reused by the next segment
     }
 
-    if (A.stage == 3 && A.cmf_part != nullptr) {
-        // every CTA of the stage's launches signals; the last one reduces each case's partials
+    if (A.stage == 3 && A.cmf_sum != nullptr) {
+        // every CTA of the stage's launches signals; the last one turns each case's sums into the shift
+        // delta = target - sum(rho u V) / sum(V), wmles/solver.py:24-29
         __shared__ bool last_cta;
-        if (tid == 0) __threadfence();
+        if (tid < 3) __threadfence();
         __syncthreads();
         if (tid == 0) last_cta = atomicAdd(A.cmf_counter, 1u) == unsigned(A.cmf_ctas - 1);
         __syncthreads();
         if (last_cta) {
-            // per case: the sum over that case's partials in slot order (the same alone or in
-            // a batch, for any chunk length, run to run) and the shift
-            // delta = target - sum(rho u V) / sum(V), wmles/solver.py:24-29
             __threadfence();
-            const volatile double* part = A.cmf_part;
-            for (int c = 0; c < A.ncases; ++c) {
+            for (int c = tid; c < A.ncases; c += NTH) {
                 const CaseDev& Cc = A.cases[c];
                 if (Cc.cmf_dir < 0) continue;
-                const int s0 = A.case_slot_start[c], s1 = A.case_slot_start[c + 1];
-                double s = 0.0;
-                for (int i = s0 + tid; i < s1; i += NTH) s += part[i];
+                double* sum = A.cmf_sum + 3 * c;
+                const double hi = __ldcg(sum);
+                // an infinite value leaves NaN in the lower bins
+                const double tot = isfinite(hi) ? hi + (__ldcg(sum + 1) + __ldcg(sum + 2)) : hi;
+                A.cmf_delta[c] = Cc.cmf_target - tot / Cc.cmf_volume;
 #pragma unroll
-                for (int off = 16; off > 0; off >>= 1) s += __shfl_down_sync(0xffffffffu, s, off);
-                __syncthreads();
-                if ((tid & 31) == 0) red[tid >> 5] = s;
-                __syncthreads();
-                if (tid == 0) {
-                    double tot = 0.0;
-                    for (int w = 0; w < NTH / 32; ++w) tot += red[w];
-                    A.cmf_delta[c] = Cc.cmf_target - tot / Cc.cmf_volume;
-                }
+                for (int m = 0; m < 3; ++m) sum[m] = 0.0;
             }
             if (tid == 0) *A.cmf_counter = 0u;
         }
@@ -1036,22 +1049,22 @@ double split_planes(long long cols, int n0, int slots, int* chunk, int* tail) {
     if (chunk) *chunk = n0;
     if (tail) *tail = 0;
     double best = 1e300;
-    for (int ic = 1; ic <= n0; ++ic) {
-        const long long waves = (cols * ((n0 + ic - 1) / ic) + slots - 1) / slots;
-        const double cost = double(waves) * (ic + SEG_PLANES);
+    for (int ic = 1, m; ic <= n0; ic = m > 1 ? (n0 + m - 2) / (m - 1) : n0 + 1) {    // the shortest for each number of chunks
+        m = (n0 + ic - 1) / ic;
+        const double cost = double((cols * m + slots - 1) / slots) * (ic + SEG_PLANES);
         if (cost < best - 1e-9) { best = cost; if (chunk) *chunk = ic; }
     }
     const long long q = slots / cols, r = slots - q * cols;
     if (q < 1 || r < 1) return best;
     const long long m = (cols + r - 1) / r;            // tail segments of the busiest tail CTA
-    for (int x = 8; x < n0 / 2; ++x) {                 // tail segments of at least 8 planes
+    for (int x = 8; x < n0 / 2 && m * (x + SEG_PLANES) < best; ++x) {      // tail segments of at least 8 planes
         const double cost = std::max((n0 - x + q - 1) / q + SEG_PLANES, m * (x + SEG_PLANES));
         if (cost < best - 1e-9) { best = cost; if (tail) *tail = x; }
     }
     return best;
 }
 
-// Tile shape of a block of n cells that may use `slots` resident CTAs.  tile >= 0: the requested
+// Tile shape of `count` blocks of n cells that may use `slots` resident CTAs together.  tile >= 0: the requested
 // shape.  Else the cheapest split of its j-k plane into equal tiles within the kernel's capacities:
 // estimated time of the launch = planes the busiest CTA marches (split_planes) x time of a
 // plane.  That time has a part that does not shrink with the tile, one thread's chain of work and
@@ -1060,7 +1073,7 @@ double split_planes(long long cols, int n0, int slots, int* chunk, int* tail) {
 // 256 x 128 x 128: FP64 8x32 663, 16x16 712, 6x32 749, 4x32 1010; float 16x32 371, 12x32 413,
 // 6x64 415, 8x32 512; on the C-grid (40 cells along k): FP64 6x40 554, 12x20 571, 5x40 600,
 // 16x16 724, 8x32 944; float 11x40 261, 8x40 265, 16x22 278, 16x32 339.
-void tile_shape(const StageOpts& o, const int n[3], int slots, int* tj, int* tk) {
+void tile_shape(const StageOpts& o, const int n[3], int count, int slots, int* tj, int* tk) {
     switch (o.tile) {
         case 0: *tj = 8; *tk = 32; return;
         case 1: *tj = 16; *tk = 16; return;
@@ -1088,7 +1101,7 @@ void tile_shape(const StageOpts& o, const int n[3], int slots, int* tj, int* tk)
                 (j + 1) * k + j * (k + 1) > L.fn || j + 3 > L.rows || k + 2 > L.kn)
                 continue;
             const double plane = fixed * full + (1.0 - fixed) * items(j, k) * (1.0 + 4.0 / k);
-            const double cost = split_planes((long long)mj * mk, n[0], slots, nullptr, nullptr) * plane;
+            const double cost = split_planes((long long)count * mj * mk, n[0], slots, nullptr, nullptr) * plane;
             if (cost < best * (1.0 - 1e-9)) { best = cost; *tj = j; *tk = k; }
         }
     }

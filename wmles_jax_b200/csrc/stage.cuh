@@ -34,7 +34,7 @@ double split_planes(long long cols, int n0, int slots, int* chunk, int* tail);
 // tile columns of the kernel variant the options select
 int stage_cap(const StageOpts& o);
 cudaError_t launch_stage(const StageArgs& A, const StageOpts& o, cudaStream_t s);
-void tile_shape(const StageOpts& o, const int n[3], int slots, int* tj, int* tk);
+void tile_shape(const StageOpts& o, const int n[3], int count, int slots, int* tj, int* tk);
 int stage_ctas_per_sm(const StageOpts& o);
 
 }  // namespace wm

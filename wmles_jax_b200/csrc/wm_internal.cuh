@@ -78,7 +78,7 @@ struct BlockDev {
     const double* met;     // WM_NMET x ncell (float64)
     const float* met32;    // WM_NMET x ncell (float32 copy for the mixed form), may be null
     int wall[6];       // view wall index of face (axis*2 + side), -1 if not wall-modelled
-    int tj, tk;        // shape of its stage tiles
+    int tj, tk;        // shape of its stage tiles in this view
     FastDiv div_nj, div_nk;   // by n[1], n[2]
     // blocks extruded along k (ext_check in geom.cu): metrics per (i, j) row and per k; else null
     const double* rows;    // N[0] x N[1] x RT_N
@@ -113,6 +113,7 @@ struct CaseDev {
     double Pr13, Pr3, kader_beta;   // Pr^(1/3), Pr^3, (3.85 Pr^(1/3) - 1.3)^2 + 2.12 ln Pr
     int cmf_dir;
     double cmf_target, cmf_volume;
+    double cmf_bin[3];     // roundings of the mass-flux sum (cmf_bins in capi.cu)
     int sponge;
     double sp_xs, sp_inv_dx, sp_sigma0, sp_invL;   // sigma = sigma0 * ramp(eta)
     unsigned int* status;  // the case's status word (WM_ST_* bits, set with atomicOr)
@@ -132,7 +133,6 @@ struct WallDev {
 struct Tile {
     int blk, j0, k0, i0, i1;   // blk: view block index
     int tj, tk;                // extents of this tile (the block's last ones may be smaller)
-    int col;                   // index of its (j,k) column in the block
 };
 
 // one case's ghost-cell program inside a view-wide gather launch
@@ -165,19 +165,17 @@ struct StageArgs {
     const CaseDev* cases;
     const WallDev* walls;
     const Tile* tiles;
-    int ntiles;
     const int* cta_first;         // CTA c runs tiles [cta_first[c], cta_first[c+1]); null: tile c
     int nctas;                    // grid size
     int stage;                    // 0: q_out = RHS; 1,2,3: SSP-RK3 stage
     int ncases;
-    const int* case_slot_start;   // ncases + 1: partial-sum slots of case c are [start[c], start[c+1])
-    double* cmf_part;             // stage 3 with constant mass flux: per (column, plane, warp) partials
+    double* cmf_sum;              // stage 3 with constant mass flux: per case the sum of rho u V in three bins
+                                  // (zero between steps: reset by the last CTA); else null
     unsigned int* cmf_counter;    // last-CTA-done counter (the last CTA resets it)
     int cmf_ctas;                 // CTAs of the stage's launches
     int ext;                      // the tiles' blocks are extruded along k
     double* cmf_delta;            // per case: constant-mass-flux shift, written by the last CTA
     const double* dt[MAX_CASES];  // per case: device time step
-    int cmf_slot_start[WM_MAX_BLOCKS];   // first partial-sum slot of each block
     StatePtrs p[WM_MAX_BLOCKS];
 };
 

@@ -20,9 +20,9 @@ waiting ones, so requests that arrive while others run join the next step.
 * Host preparation (lowering, ghost programs, initial state) runs on builder threads,
   overlapping the GPU steps; graph captures and device-side case construction exclude each
   other.
-* Results do not depend on the mix: per-case reductions run over that case's own cells in
-  a fixed order and its stage tiles are fixed at construction, so a case advanced in any
-  batch is bit-identical to the same case advanced alone with ``Solver.step``.
+* Results do not depend on the mix: per-case reductions run over that case's own cells and are
+  exact in any order, so a case advanced in any batch is bit-identical to the same case
+  advanced alone with ``Solver.step``, although the batch cuts its blocks into other tiles.
 * Time-to-result is measured from the request's arrival to the moment the host sees the
   device finish the request's last step (an event per step, at most six steps in flight).
 * Failure: every step also copies the members' status words (non-finite state, density or
