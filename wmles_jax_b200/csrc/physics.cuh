@@ -291,10 +291,14 @@ __device__ __forceinline__ double spalding_utau(double kappa, double ekb, int n_
     const double Reh = h * U * rho_w / mu_w;
     // F has one root (dF > 0 everywhere), so that every start that settles ends at the same u+.  Over
     // Reh = 625, where the reference starts from 25 whatever the root, the logarithmic layer's estimate
-    // (Reh = u+ y+ with u+ = 18) saves about four iterations; with fewer than 30 iterations, where the
-    // reference's start might not settle and its last iterate is the answer, that start is kept
+    // (Reh = u+ y+ with u+ = 18) saves about four iterations.  Only where the reference's own start
+    // settles, as its last iterate is the answer otherwise: from above the root an iteration lowers
+    // kappa u+ by at most one, from 25 or, after an overshoot, 50 to 100, some 50 kappa iterations in all (29
+    // at kappa = 0.6, counted over B and Reh); and where rounding leaves both starts at one u+ (ekb, the size
+    // of F's terms over their sum near the wall, at most 100: B above -11 at kappa = 0.41)
     double up = fmin(fmax(sqrt(Reh), 1.0), 25.0);
-    if (n_iter >= 30 && Reh > 625.0 && Reh < 1e12) up = fmin(fmax(log(Reh / (18.0 * ekb)) / kappa, 1.0), 100.0);
+    if (n_iter >= 30 && kappa > 0.0 && kappa <= 0.6 && ekb <= 100.0 && Reh > 625.0 && Reh < 1e12)
+        up = fmin(fmax(log(Reh / (18.0 * ekb)) / kappa, 1.0), 100.0);
     double last = 0.0;
     *moving = false;
     for (int it = 0; it < n_iter; ++it) {
