@@ -140,6 +140,13 @@ __device__ __forceinline__ void albada2(R a, R b, R c, R& l, R& r) {
     }
 }
 
+// a / b from inv, 1 / b to a few units in the last place: one correction by the remainder, so that the quotient
+// is rounded about as a division rounds it
+__device__ __forceinline__ double quotient(double a, double b, double inv) {
+    const double q = a * inv;
+    return fma(fma(-q, b, a), inv, q);
+}
+
 // HLLC flux times |S|, wmles/schemes.py:108-137
 template <int FACE, typename R>
 __device__ __forceinline__ void hllc_flux(const R wl[5], const R wr[5], R Sx, R Sy, R Sz, R gamma,
@@ -153,7 +160,10 @@ __device__ __forceinline__ void hllc_flux(const R wl[5], const R wr[5], R Sx, R 
     const R unl = dot_s<FACE>(ul, vl, wlz, nx, ny, nz);
     const R unr = dot_s<FACE>(ur, vr, wrz, nx, ny, nz);
     // FP64: 1 / rl and 1 / rr from 1 / (rl rr), later 1 / (s - un) and 1 / (s - ss) from their
-    // product's: four divisions a face instead of seven, of some 30 instructions each
+    // product's: four divisions a face instead of seven, of some 30 instructions each.  The two quotients
+    // that the flux is proportional to are corrected (uncorrected, the residual's error against extended precision
+    // was 14-20 % larger than with divisions; the other two, under a root and beside a larger term,
+    // make no difference to it)
     const R irr = D ? R(1) / (rl * rr) : R(0), il = rr * irr, ir = rl * irr;
     const R cl = wm_sqrt(D ? gamma * pl * il : gamma * pl / rl), cr = wm_sqrt(D ? gamma * pr * ir : gamma * pr / rr);
     const R sL = fmin(unl - cl, unr - cr), sR = fmax(unl + cl, unr + cr);
@@ -175,10 +185,10 @@ __device__ __forceinline__ void hllc_flux(const R wl[5], const R wr[5], R Sx, R 
         const R s = left ? sL : sR;
         R f, e;
         if constexpr (D) {
-            const R q = R(1) / ((s - un) * (s - ss));
+            const R a = s - un, b = s - ss, q = R(1) / (a * b), ra = r * a;
             const R iro = left ? il : ir;
-            f = r * (s - un) * ((s - un) * q);
-            e = E * iro + (ss - un) * (ss + p * iro * ((s - ss) * q));
+            f = quotient(ra, b, a * q);
+            e = quotient(E, r, iro) + (ss - un) * (ss + p * (iro * (b * q)));
         } else {
             f = r * (s - un) / (s - ss);
             e = E / r + (ss - un) * (ss + p / (r * (s - un)));
