@@ -7,8 +7,9 @@ on the grid extents (partial tiles at the j/k edges, waves of CTAs over the SMs)
 precision (registers and shared memory decide CTAs per SM) and on the scheme.  ``tune``
 measures it: for each candidate tile it builds the cases with that tile, advances them
 together (one batched step, as the server runs them) and times the steps with CUDA events;
-the fastest tile is stored in a JSON cache keyed by GPU name, precision, scheme, SGS model
-and the block extents of the workload, so each workload is tuned once per machine.
+the fastest tile is stored in a JSON cache keyed by GPU name, precision, scheme, SGS model,
+the extents and kind (extruded along k or not: different kernels) of the workload's blocks and
+the library's contents, so each workload is tuned once per machine and build.
 
 The tile shape does not change the physics; ids 0-2 and 3 / -1 of the mixed form are different
 kernel instances, whose results agree to round-off, not bitwise.  A server therefore
@@ -16,6 +17,7 @@ fixes one tile for all its cases (``Server(tile="auto")`` tunes it over its grid
 serving).
 """
 import copy
+import hashlib
 import json
 import os
 import threading
@@ -35,10 +37,38 @@ def cache_path():
     return os.path.join(os.path.expanduser("~"), ".cache", "wmles_jax_b200", "tiles.json")
 
 
-def workload_key(dims, precision, scheme, sgs, device_name):
-    """Cache key of a workload: the sorted multiset of block extents plus the options."""
-    ext = sorted("x".join(str(int(n)) for n in d) for d in dims)
-    return f"{device_name}|{precision}|{scheme}|{sgs}|{','.join(ext)}"
+def workload_key(dims, precision, scheme, sgs, device_name, extruded=None, kernels=None):
+    """Cache key of a workload: the sorted multiset of block extents (marked "e" where ``extruded``
+    says so, one flag per block) plus the options and the kernels' version."""
+    ext = sorted("x".join(str(int(n)) for n in d) + ("e" if extruded is not None and extruded[i] else "")
+                 for i, d in enumerate(dims))
+    return f"{device_name}|{precision}|{scheme}|{sgs}|{','.join(ext)}" + (f"|{kernels}" if kernels else "")
+
+
+def library_version(path=None):
+    """Digest of the kernel library: an answer timed with other kernels is not an answer."""
+    from . import _native
+    with open(path or _native.LIB_PATH, "rb") as f:
+        return hashlib.file_digest(f, "sha1").hexdigest()[:12]
+
+
+def is_extruded(block):
+    """Whether the block's nodes are one (i, j) surface extruded along k (the library decides by
+    the metrics; for the key it is enough that like grids get like marks)."""
+    x = block.x_int
+    return bool((x[:2] == x[:2, :, :, :1]).all() and (x[2] == x[2, :1, :1]).all())
+
+
+def lookup(key, precision, tiles=None, path=None):
+    """The cached (tile, timings) of a workload, or None.  Without an explicit choice of tiles, an
+    entry must have timed every candidate."""
+    hit = load_cache(path).get(key)
+    if hit is None:
+        return None
+    timings = {int(k): v for k, v in hit["ms_per_step"].items()}
+    if tiles is None and not set(CANDIDATES[precision]) <= set(timings):
+        return None
+    return int(hit["tile"]), timings
 
 
 def load_cache(path=None):
@@ -84,9 +114,10 @@ def key_for(cases, precision):
     import torch
     from .sgs import make_sgs
     mesh0, _, kw0, _ = cases[0]
-    dims = [tuple(b.n) for mesh, _, _, _ in cases for b in mesh.blocks]
+    blocks = [b for mesh, _, _, _ in cases for b in mesh.blocks]
     sgs = make_sgs(kw0.get("sgs", "vreman"), **(kw0.get("sgs_kwargs") or {})).name
-    return workload_key(dims, precision, _scheme_name(kw0["scheme"]), sgs, torch.cuda.get_device_name())
+    return workload_key([tuple(b.n) for b in blocks], precision, _scheme_name(kw0["scheme"]), sgs,
+                        torch.cuda.get_device_name(), [is_extruded(b) for b in blocks], library_version())
 
 
 def tune(cases, precision="mixed", tiles=None, steps=20, warmup=3, use_cache=True, path=None):
@@ -97,9 +128,9 @@ def tune(cases, precision="mixed", tiles=None, steps=20, warmup=3, use_cache=Tru
     from .serving import Batch
     key = key_for(cases, precision)
     if use_cache:
-        hit = load_cache(path).get(key)
+        hit = lookup(key, precision, tiles, path)
         if hit is not None:
-            return int(hit["tile"]), {int(k): v for k, v in hit["ms_per_step"].items()}
+            return hit
     tiles = CANDIDATES[precision] if tiles is None else tuple(tiles)
     # host lowering and initial states once; device cases per tile
     prepared, q0 = [], []
