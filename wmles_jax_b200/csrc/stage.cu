@@ -66,10 +66,10 @@ struct StageLayout {
     // to spare: channel, three steps, float 3681 -> 3945, FP64 6411 -> 6461, so one by one there
     static constexpr int GV = EXT ? 1 : sizeof(R) == 4 ? 4 : SCHEME == WM_SCHEME_HYBRID ? 1 : 2;
     static constexpr int NGS = GV == 4 ? 16 : (SCHEME == WM_SCHEME_HYBRID) ? 15 : 14;
-    // FP64, one CTA per SM: a fifth primitive slot (the shared memory is there), so plane
-    // i+2 is converted while the gradient records of plane i are computed, by the warps that
-    // have no record to compute, and a plane takes two barriers instead of three.  The float
-    // form has a record for nearly every thread and keeps three phases.
+    // FP64: plane i+2 is converted while the gradient records of plane i are computed, by the warps that
+    // have no record to compute, and a plane takes two barriers instead of three.  It goes into the slot of plane
+    // i-2, whose records the columns have copied (hp).  The float form has a record for nearly every thread and
+    // keeps three phases.
     static constexpr bool FUSE = sizeof(R) == 8;
     static constexpr int NSLOT = 4;
     static constexpr int HP_N = 6;
@@ -143,7 +143,7 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
 template <int FACE, typename R, class GL, class GR>
 __device__ __forceinline__ void viscous_flux(const R* pl, const R* pr, int s, GL gL, GR gR, R Sx, R Sy, R Sz,
                                              R e0, R e1, R e2, R idist, R V[4]) {
-    // a record's components one by one, or GW at a time (StageLayout::GW)
+    // a record's components one by one, or GW at a time (StageLayout::GV)
     constexpr int GW = sizeof(decltype(gL(0))) / sizeof(R);
     R gf[12], sum[GW > 1 ? 16 : 1];
     if constexpr (GW > 1) {
@@ -739,6 +739,8 @@ __device__ __forceinline__ void stage_segment(const StageArgs& A, const StageOpt
         if constexpr (LY::PING) gs = gs == gs0 ? gs0 + NGS * GN : gs0;
     };
     auto faces = [&](int ip) {
+        // in two rounds, the threads without columns take faces [0, 2 XTRA), the others the CAP after those
+        static_assert(XROUNDS == 1 || FN <= NTH + XTRA, "the strides below leave out faces beyond the first rounds");
         if (ip < i0 || ip >= i1) return;
         const int f0 = tid < CAP ? tid + XROUNDS * XTRA : tid - CAP;
         const int step0 = tid < CAP || XROUNDS == 1 ? NTH + (XROUNDS - 1) * XTRA : XTRA;
