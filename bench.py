@@ -41,13 +41,13 @@ N_CFG2 = (256, 128, 128)
 # DRAM bytes (read + write) per stage-kernel launch per interior cell, mean of the three RK
 # stages, from one ncu capture of the same kernel on a 128^3 case of this workload; scaled
 # by the cell count for the roofline's `traffic`
-TRAFFIC_PER_CELL = {"fp64": 130.0, "mixed": 126.0}
+TRAFFIC_PER_CELL = {"fp64": 130.0, "mixed": 125.0}
 # FP64 work per interior cell per stage-kernel launch (FP64 form, mean of the three RK
-# stages), from one ncu capture of the same kernel on a 128^3 case of this workload: DADD 233.4,
-# DMUL 300.1, DFMA 268.3 thread instructions, i.e. 1070 flop (an FMA counts two) in 802
+# stages), from one ncu capture of the same kernel on a 128^3 case of this workload: DADD 239.9,
+# DMUL 300.5, DFMA 268.0 thread instructions, i.e. 1076 flop (an FMA counts two) in 808
 # FP64-pipe instructions
-FP64_FLOP_PER_CELL = 1070.0
-FP64_INST_PER_CELL = 802.0
+FP64_FLOP_PER_CELL = 1076.0
+FP64_INST_PER_CELL = 808.0
 # nominal FP64 rate of a B200: 148 SMs x 64 FP64 lanes x 1.965 GHz (x 2 flop per FMA)
 FP64_PEAK_INST = 148 * 64 * 1.965e9
 FP64_PEAK_TFLOPS = 2 * FP64_PEAK_INST / 1e12
