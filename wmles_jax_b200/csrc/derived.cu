@@ -187,7 +187,7 @@ cudaError_t launch_derived(DerivedArgs A, const int n[3], cudaStream_t s) {
     const int tk = 1 << A.lt, tj = DV_NT >> A.lt;
     A.ktiles = (n[2] + tk - 1) / tk;
     const int tiles = (n[1] + tj - 1) / tj * A.ktiles;
-    const int chunks = std::min(n[0], std::max((n[0] + 31) / 32, 148 * DV_CPS / tiles));
+    const int chunks = std::min(n[0], std::max((n[0] + 31) / 32, CHIP_SMS * DV_CPS / tiles));
     A.planes = (n[0] + chunks - 1) / chunks;
     derived_kernel<<<dim3(tiles, (n[0] + A.planes - 1) / A.planes), DV_NT, 0, s>>>(A);
     return cudaGetLastError();

@@ -1074,7 +1074,8 @@ double split_planes(long long cols, int n0, int slots, int* chunk, int* tail) {
 // cost some more (whole 128-byte lines).  Fitted to stage times (us per launch) on the channel
 // 256 x 128 x 128: FP64 8x32 663, 16x16 712, 6x32 749, 4x32 1010; float 16x32 371, 12x32 413,
 // 6x64 415, 8x32 512; on the C-grid (40 cells along k): FP64 6x40 554, 12x20 571, 5x40 600,
-// 16x16 724, 8x32 944; float 11x40 261, 8x40 265, 16x22 278, 16x32 339.
+// 16x16 724, 8x32 944; float 11x40 261, 8x40 265, 16x22 278, 16x32 339.  Looked at on 120 batches of 3 to 96
+// channels of 8^3 to 192 x 96 x 96, both forms and kinds: 0.74-1.01 of the fixed shape's time where both were timed.
 void tile_shape(const StageOpts& o, const int n[3], int count, int slots, int* tj, int* tk) {
     switch (o.tile) {
         case 0: *tj = 8; *tk = 32; return;

@@ -94,10 +94,10 @@ __global__ void __launch_bounds__(PS_NT, PS_CPS) plane_stats_kernel(const __grid
     if (threadIdx.x == 0) A.counter[jj] = 0u;
 }
 
-// chunks per plane: one wave of CTAs on 148 SMs (a constant, so that the order of the sums does
+// chunks per plane: one wave of CTAs on CHIP_SMS (a constant, so that the order of the sums does
 // not depend on the device), at most PS_CHUNKS and one plane of cells each
 int plane_chunks(int ni, int nj) {
-    return std::max(1, std::min({PS_CHUNKS, ni, 148 * PS_CPS / std::max(1, nj)}));
+    return std::max(1, std::min({PS_CHUNKS, ni, CHIP_SMS * PS_CPS / std::max(1, nj)}));
 }
 
 cudaError_t launch_plane_stats(const PlaneStatsArgs& A, int nj, cudaStream_t s) {

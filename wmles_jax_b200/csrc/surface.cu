@@ -331,11 +331,11 @@ __global__ void __launch_bounds__(SURF_NT, 4) surface_kernel(const __grid_consta
 
 cudaError_t launch_surface(SurfaceArgs& A, cudaStream_t s) {
     A.g_ctas = (A.G.total + SURF_NT - 1) / SURF_NT;
-    // wall faces per CTA: as few as spread them over the chip (148 SMs; a face is a chain of FP64 operations
+    // wall faces per CTA: as few as spread them over the chip (a face is a chain of FP64 operations
     // and the warps of one SM share its FP64 units), in whole warps, at most one per thread.  Channel
     // 32 x 32 x 16 (1024 faces, 32 per CTA instead of 256), with the Newton iteration's start and stop:
     // 12.4 -> 9.2 us a launch
-    const int spread = (A.W.nwalls * A.W.max_faces / 148 + 31) / 32 * 32;
+    const int spread = (A.W.nwalls * A.W.max_faces / CHIP_SMS + 31) / 32 * 32;
     A.w_nt = std::max(32, std::min(SURF_NT, spread));
     A.w_per = A.W.nwalls ? (A.W.max_faces + A.w_nt - 1) / A.w_nt : 0;
     A.w_ctas = A.w_per * A.W.nwalls;

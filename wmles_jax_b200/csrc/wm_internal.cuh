@@ -53,6 +53,9 @@ inline cudaError_t launch_chained(void (*kernel)(P...), unsigned ctas, unsigned 
 
 constexpr int MAX_CASES = WM_MAX_BLOCKS;   // a case has at least one block
 
+// SMs of a B200: the constant where a rule for spreading work (or the order of a sum) must not depend on the device
+constexpr int CHIP_SMS = 148;
+
 // x / d of a divisor known at set-up, for 0 <= x < 2^31: (x mul) >> shift with mul = ceil(2^shift / d),
 // shift = 31 + ceil(log2 d) (mul < 2^33 x 2^31 fits 64 bits; exact for 31-bit x)
 struct FastDiv {
